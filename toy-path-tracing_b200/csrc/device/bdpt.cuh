@@ -312,18 +312,13 @@ __device__ __forceinline__ void camera_step(const DevRender& S, const RenderLaun
     return;
   }
   if (S.d.num_extra_lights > 0) {  // direct_non_area_light_contribution
-    float us0, us1;
-    ps.sample_2d(vertex_dim(depth, kOffSurface), us0, us1);
-    const float u_tree = ps.sample_1d(vertex_dim(depth, kOffTree));
-    const float u_cat = S.d.num_cat > 1 ? ps.sample_1d(vertex_dim(depth, kOffCategory)) : 0.0f;
-    nee = prepare_direct<true, kDirectBdptNonArea>(S, m, v, u_cat, u_tree, us0, us1, dp);
+    nee = prepare_direct<true, kDirectBdptNonArea>(S, m, v, ps, depth, dp);
     if (nee) dp.contrib = c.beta * dp.contrib;
   }
-  float ud0, ud1;
-  ps.sample_2d(vertex_dim(depth, kOffDir), ud0, ud1);
-  const float u_lobe = m.kind == kDevOpenPbr ? ps.sample_1d(vertex_dim(depth, kOffLobe)) : 0.0f;
-  float ux[4];
-  extra_randoms(S.d, m, ps, depth, ux);
+  float ud0, ud1, u_lobe = 0.0f, ux[4];
+  if (m.kind == kDevOpenPbr) ps.sample_2d_1d(vertex_dim(depth, kOffDir), vertex_dim(depth, kOffLobe), ud0, ud1, u_lobe);
+  else ps.sample_2d(vertex_dim(depth, kOffDir), ud0, ud1);
+  extra_randoms(S.d, m, v, ps, depth, ux);
   MatSample s;
   if (!material_sample_rev(S, m, v, u_lobe, ud0, ud1, ux, false, s)) {
     c.alive = false;
@@ -470,11 +465,10 @@ __device__ __forceinline__ void light_step(const DevRender& S, const PathSampler
     l.alive = false;
     return;
   }
-  float ud0, ud1;
-  ps.sample_2d(vertex_dim(depth, kOffDir), ud0, ud1);
-  const float u_lobe = m.kind == kDevOpenPbr ? ps.sample_1d(vertex_dim(depth, kOffLobe)) : 0.0f;
-  float ux[4];
-  extra_randoms(S.d, m, ps, depth, ux);
+  float ud0, ud1, u_lobe = 0.0f, ux[4];
+  if (m.kind == kDevOpenPbr) ps.sample_2d_1d(vertex_dim(depth, kOffDir), vertex_dim(depth, kOffLobe), ud0, ud1, u_lobe);
+  else ps.sample_2d(vertex_dim(depth, kOffDir), ud0, ud1);
+  extra_randoms(S.d, m, v, ps, depth, ux);
   MatSample s;
   if (!material_sample_rev(S, m, v, u_lobe, ud0, ud1, ux, true, s)) {
     l.alive = false;

@@ -217,16 +217,25 @@ __device__ __forceinline__ uint32_t aux_from_seed(const PathSamplerDev& ps, int 
   return pcg_state_transition(ps.aux_rng_seed(depth < 0 ? 0x80000000u : vertex_dim((uint32_t)depth, kOffAuxSeed)));
 }
 
-// MaterialSampleRandoms::u_extra0..3 (offsets 9-12), drawn only for a
-// dispersive material (the only reader); zeros otherwise.
-__device__ __forceinline__ void extra_randoms(const DevRenderData& d, const DevMaterialRec& m,
+// MaterialSampleRandoms::u_extra0..3 (offsets 9-12), zeros where no one reads
+// them: they choose wavelengths of a dispersive solid's transmission, entered
+// from the front by a path without a wavelength lock -- u_extra0 at a smooth
+// surface, all four at a rough one.
+__device__ __forceinline__ void extra_randoms(const DevRenderData& d, const DevMaterialRec& m, const Vertex& v,
                                               const PathSamplerDev& ps, uint32_t depth, float* ux) {
   ux[0] = ux[1] = ux[2] = ux[3] = 0.0f;
-  if (m.kind != kDevOpenPbr || !(d.openpbr[m.openpbr].flags & kOpbrDisp)) return;
-  ux[0] = ps.sample_1d(vertex_dim(depth, kOffExtra0));
-  ux[1] = ps.sample_1d(vertex_dim(depth, kOffExtra1));
-  ux[2] = ps.sample_1d(vertex_dim(depth, kOffExtra2));
-  ux[3] = ps.sample_1d(vertex_dim(depth, kOffExtra3));
+  if (m.kind != kDevOpenPbr || v.lock >= 0.0f || !v.front) return;
+  const uint32_t flags = d.openpbr[m.openpbr].flags;
+  if (!(flags & kOpbrDisp) || (flags & kOpbrThinWalled)) return;
+  if (!(flags & kOpbrTransRough)) {
+    ux[0] = ps.sample_1d(vertex_dim(depth, kOffExtra0));
+    return;
+  }
+  const float4 r = ps.sample_1d4(vertex_dim(depth, kOffExtra0));
+  ux[0] = r.x;
+  ux[1] = r.y;
+  ux[2] = r.z;
+  ux[3] = r.w;
 }
 
 // Material::sample for the BSDF materials in scope, with the vertex's
@@ -234,13 +243,14 @@ __device__ __forceinline__ void extra_randoms(const DevRenderData& d, const DevM
 __device__ __forceinline__ bool material_sample(const DevRender& S, const DevMaterialRec& m, const Vertex& v,
                                                 const PathSamplerDev& ps, uint32_t depth, BsdfSampleOut& s) {
   float ud0, ud1;
-  ps.sample_2d(vertex_dim(depth, kOffDir), ud0, ud1);
   if (m.kind == kDevOpenPbr) {
-    const float u_lobe = ps.sample_1d(vertex_dim(depth, kOffLobe));
+    float u_lobe;
+    ps.sample_2d_1d(vertex_dim(depth, kOffDir), vertex_dim(depth, kOffLobe), ud0, ud1, u_lobe);
     float ux[4];
-    extra_randoms(S.d, m, ps, depth, ux);
+    extra_randoms(S.d, m, v, ps, depth, ux);
     return openpbr_sample(S.d, m.openpbr, v, u_lobe, ud0, ud1, ux, s);
   }
+  ps.sample_2d(vertex_dim(depth, kOffDir), ud0, ud1);
   return lambert_sample(m, v, ud0, ud1, s);
 }
 
@@ -532,14 +542,21 @@ struct DirectPrep {
 // MIS weight; kDirectBdptNonArea: BDPT's direct_non_area_light_contribution
 // (integrator/bdpt.rs:396-464), zero when the sampled light is an area light.
 enum DirectMode : int { kDirectMis = 0, kDirectBdptNonArea = 1 };
+//
+// The vertex's light randoms (category, tree, surface) are drawn here, each
+// only where it is read: one category takes any u, directional lights read
+// nothing more, and an OpenPBR vertex in a scene with area lights alone (no
+// light-tree query) draws none.
 template <bool LIGHTS, int MODE = kDirectMis>
 __device__ __forceinline__ bool prepare_direct(const DevRender& S, const DevMaterialRec& m, const Vertex& v,
-                                               float u_cat, float u_tree, float us0, float us1, DirectPrep& out,
+                                               const PathSamplerDev& ps, uint32_t depth, DirectPrep& out,
                                                bool nee = false) {
   float cat_pmf;
   uint32_t cat;
+  float us0 = 0.0f, us1 = 0.0f;
   if (LIGHTS) {
     if (S.d.num_cat == 0) return false;  // LightSampler::sample_category: no category
+    const float u_cat = S.d.num_cat > 1 ? ps.sample_1d(vertex_dim(depth, kOffCategory)) : 0.0f;
     cat = sample_category(S.d, u_cat, cat_pmf);
   } else {
     if (!S.d.has_tree) return false;
@@ -558,7 +575,8 @@ __device__ __forceinline__ bool prepare_direct(const DevRender& S, const DevMate
     if (q.rho <= 0.0f) return false;
     q.p = v.p;
     q.n = v.ns;
-    float leaf_pmf;
+    float leaf_pmf, u_tree;
+    ps.sample_2d_1d(vertex_dim(depth, kOffSurface), vertex_dim(depth, kOffTree), us0, us1, u_tree);
     const uint32_t leaf = sample_light_tree(S.d.ltree, S.d.ltree_root, q, u_tree, leaf_pmf);
     if (leaf == 0xFFFFFFFFu) return false;
     const uint32_t li_inst = __ldg(&S.d.ltree[leaf].leaf_instance), li_tri = __ldg(&S.d.ltree[leaf].leaf_triangle);
@@ -573,6 +591,7 @@ __device__ __forceinline__ bool prepare_direct(const DevRender& S, const DevMate
     }
     sel = cat_pmf * leaf_pmf;
   } else if (cat == kCatEnv) {
+    ps.sample_2d(vertex_dim(depth, kOffSurface), us0, us1);
     if (!sample_li_env(S.d, us0, us1, nee, li)) return false;
     delta = false;
     sel = cat_pmf;

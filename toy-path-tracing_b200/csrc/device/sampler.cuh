@@ -47,15 +47,20 @@ __device__ __forceinline__ uint64_t left_shift_2(uint64_t v) {
   return v;
 }
 
-// zsobol.rs:98-171 generator matrices, rows indexed by input bit.
-__constant__ uint16_t c_sobol_dirs[3][16] = {
-    {0xFFFF, 0x5555, 0x3333, 0x1111, 0x0F0F, 0x0505, 0x0303, 0x0101, 0x00FF, 0x0055, 0x0033, 0x0011, 0x000F,
-     0x0005, 0x0003, 0x0001},
-    {0xAA09, 0x7706, 0x3903, 0x1601, 0x09AA, 0x0677, 0x0339, 0x0116, 0x00A3, 0x0071, 0x003A, 0x0017, 0x0009,
-     0x0006, 0x0003, 0x0001},
-    {0xA0C3, 0x4041, 0x302D, 0x101E, 0x0B67, 0x079A, 0x02A4, 0x011B, 0x00C9, 0x0045, 0x002E, 0x001F, 0x000A,
-     0x0004, 0x0003, 0x0001},
-};
+// zsobol.rs:98-171, the first two generator matrices (no draw is wider than
+// 2D).  Dimension 0 reverses the bits.  Dimension 1 is the Pascal matrix: input
+// bit i feeds output bit j iff i & j == 0, so the output is the GF(2) sum over
+// the subsets of ~j: four shift-and-xor steps, then a bit reversal (~j).
+__device__ __forceinline__ uint32_t sobol_reversed_0(uint32_t index16) { return __brev(index16) >> 16; }
+__device__ __forceinline__ uint32_t sobol_reversed_1(uint32_t index16) {
+  uint32_t z = index16;
+  z ^= (z & 0x5555u) << 1;
+  z ^= (z & 0x3333u) << 2;
+  z ^= (z & 0x0F0Fu) << 4;
+  z ^= (z & 0x00FFu) << 8;
+  return __brev(z) >> 16;
+}
+
 // zsobol.rs:238-263: the 24 permutations of a base-4 digit, one byte each
 // (2 bits per digit: permutation p maps digit d to (byte_p >> 2d) & 3), packed
 // into three 64-bit immediates so a per-lane index costs ALU work instead of a
@@ -69,13 +74,82 @@ __device__ __forceinline__ uint32_t perm_digit(uint32_t p, uint32_t digit) {
   return (byte >> (2u * digit)) & 3u;
 }
 
-__device__ __forceinline__ uint32_t sobol_reversed(uint32_t index16, int dim) {
-  if (dim == 0) return __brev(index16) >> 16;
-  uint32_t s = 0;
+// The index permutation for Morton indices of at most 32 bits (image side^2 x
+// spp up to 2^32: 1080p at 1,024 spp, 4096^2 at 256), in 32-bit arithmetic.
+// The draws are most of a shading vertex's instructions (a 256 x 256 x 64 image
+// has 11 digits per draw, four to six draws per vertex), so the digit step is
+// written for instruction count; its value is mix_bits' bit for bit:
+//  - `higher` is below 2^30, so bit 31 and the high word of higher ^ dim_hash
+//    are the dimension's: the first xor-shift and the high word's share of the
+//    first product are per-dimension constants (DimHash);
+//  - bits 24.. of the mixed value modulo 24 = 8 (bits 27.. mod 3) + bits 24-26:
+//    256 = 1 (mod 3), so a byte sum (dp4a) leaves at most 2,071 to reduce;
+//  - table T_d holds permutation p's image of digit d in bits 2p, and
+//    T_3 = T_0 ^ T_1 ^ T_2 (a permutation's images are 0..3), so a digit picks
+//    its table with two masked xors; the table serves every dimension drawn.
+// Measured against the 64-bit digit loop (a 64-bit modulo by 24 and a 64-bit
+// variable shift per digit), with draws nobody reads left out: Cornell box
+// 256 x 256 x 64 11.71 -> 10.44 ms, the 2.1M-triangle scene 1080p x 16
+// 115.8 -> 106.9 ms.
+struct DimHash {
+  uint32_t x, k;
+};
+constexpr uint32_t kMix1Lo = 0x728ea185u, kMix1Hi = 0x7fb5d329u, kMix2Lo = 0xbc2dd44du, kMix2Hi = 0x81dadef4u;
+__device__ __forceinline__ DimHash dim_hash32(uint32_t dimension) {
+  const uint64_t h = 0x55555555ull * (uint64_t)dimension;
+  const uint32_t lo = (uint32_t)h, hi = (uint32_t)(h >> 32);
+  return DimHash{lo ^ ((hi << 1) | (lo >> 31)), (hi ^ (hi >> 31)) * kMix1Lo};
+}
+// mix_bits(higher ^ dim_hash) for higher < 2^31: low and high word
+__device__ __forceinline__ void mix_bits32(uint32_t higher, DimHash h, uint32_t& lo, uint32_t& hi) {
+  const uint32_t v = higher ^ h.x;
+  const uint64_t p = (uint64_t)v * kMix1Lo + ((uint64_t)h.k << 32);
+  const uint32_t p_lo = (uint32_t)p, p_hi = (uint32_t)(p >> 32) + v * kMix1Hi;
+  const uint32_t v_lo = p_lo ^ ((p_hi << 5) | (p_lo >> 27)), v_hi = p_hi ^ (p_hi >> 27);
+  const uint64_t q = (uint64_t)v_lo * kMix2Lo;
+  hi = (uint32_t)(q >> 32) + v_lo * kMix2Hi + v_hi * kMix2Lo;
+  lo = (uint32_t)q ^ (hi >> 1);
+}
+template <int N>
+__device__ __forceinline__ void sample_index32(uint32_t morton, uint32_t log2_spp, uint32_t n_digits,
+                                               const uint32_t (&dim)[N], uint32_t (&out)[N]) {
+  DimHash h[N];
 #pragma unroll
-  for (int i = 0; i < 16; ++i)
-    if (index16 & (1u << i)) s ^= c_sobol_dirs[dim - 1][i];
-  return s;
+  for (int k = 0; k < N; ++k) {
+    h[k] = dim_hash32(dim[k]);
+    out[k] = 0;
+  }
+  const uint32_t odd = log2_spp & 1u;
+  uint32_t shift = 2u * n_digits - odd;  // bits of the index not yet permuted
+  // the top digit has no digits above it: `higher` starts at 0, and the shift
+  // below never reaches 32
+  uint32_t higher = 0;
+#pragma unroll 2
+  for (; shift > odd; shift -= 2u) {
+    const uint32_t rest = morton >> (shift - 2u);
+    const uint32_t m1 = 0u - (rest & 1u), m2 = 0u - ((rest >> 1) & 1u);
+    const uint32_t t_lo = 0xaa555000u ^ (m1 & 0xafaf5fa5u) ^ (m2 & 0x7679b6deu);
+    const uint32_t t_hi = 0x0000fffau ^ (m1 & 0x0000f5a5u) ^ (m2 & 0x00009edeu);
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      uint32_t lo, hi;
+      mix_bits32(higher, h[k], lo, hi);
+      const uint32_t s = __dp4a(hi, 0x02020202u, lo >> 27);
+      const uint32_t q = (s * 0x5556u) >> 16;  // s / 3
+      // halfword s % 3 of the table, then pair (bits 24-26) of its eight
+      const uint32_t half = __byte_perm(t_lo, t_hi, s * 0x22u + 0x10u - q * 0x66u);
+      out[k] = out[k] * 4u + ((half >> ((lo >> 23) & 14u)) & 3u);
+    }
+    higher = rest;
+  }
+  if (odd) {
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      uint32_t lo, hi;
+      mix_bits32(morton >> 1, h[k], lo, hi);
+      out[k] = out[k] * 2u + ((morton ^ lo) & 1u);
+    }
+  }
 }
 
 // IndexSampler (zsobol.rs:206-285) + PathSampler (path_sampler.rs:146-250)
@@ -109,32 +183,96 @@ struct PathSamplerDev {
     return out;
   }
 
-  __device__ __noinline__ void sobol(uint32_t dimension, int depth, float* out) const {
-    const uint64_t si = sample_index(dimension);
-    const uint32_t index = (uint32_t)si ^ (uint32_t)(si >> 32);
-    const uint64_t sb = mix_bits(((uint64_t)this->seed << 32) | (uint64_t)dimension);  // seed_for_dimension
-    const uint32_t seed = (uint32_t)sb ^ (uint32_t)(sb >> 32);
-    const uint32_t idx = lk_permutation(__brev(index), seed);
-    for (int d = 0; d < depth; ++d) {
-      const uint32_t sob = sobol_reversed(idx >> 16, d);
-      const uint32_t r = (8u * (uint32_t)d) & 31u;
-      const uint32_t rot = r == 0 ? seed : ((seed >> r) | (seed << (32u - r)));
-      out[d] = uint_to_float(__brev(lk_permutation(sob, rot)));
+  __device__ __forceinline__ bool narrow() const { return 2u * n_base4_digits - (log2_spp & 1u) <= 32u; }
+
+  // sample_index of N dimensions, its words folded by xor
+  template <int N>
+  __device__ __forceinline__ void folded_indices(const uint32_t (&dim)[N], uint32_t (&index)[N]) const {
+    if (narrow()) {
+      sample_index32<N>((uint32_t)morton, log2_spp, n_base4_digits, dim, index);
+    } else {
+#pragma unroll
+      for (int k = 0; k < N; ++k) {
+        const uint64_t si = sample_index(dim[k]);
+        index[k] = (uint32_t)si ^ (uint32_t)(si >> 32);
+      }
     }
   }
-  __device__ __forceinline__ float sample_1d(uint32_t dim) const {
-    float v[1];
-    sobol(dim, 1, v);
-    return v[0];
+  // the Owen-scrambled Sobol point of a dimension at a folded index
+  template <bool SECOND>
+  __device__ __forceinline__ void point(uint32_t dimension, uint32_t index, float& a, float& b) const {
+    const uint64_t sb = mix_bits(((uint64_t)this->seed << 32) | (uint64_t)dimension);  // seed_for_dimension
+    const uint32_t seed = (uint32_t)sb ^ (uint32_t)(sb >> 32);
+    const uint32_t idx = lk_permutation(__brev(index), seed) >> 16;
+    a = uint_to_float(__brev(lk_permutation(sobol_reversed_0(idx), seed)));
+    if (SECOND) b = uint_to_float(__brev(lk_permutation(sobol_reversed_1(idx), (seed >> 8) | (seed << 24))));
   }
+  // Out of line and by value: a draw is some 400 instructions, and a shading
+  // vertex makes several; the kernels keep one copy of each form.
+  static __device__ __noinline__ float draw_1(PathSamplerDev s, uint32_t dim) {
+    const uint32_t d[1] = {dim};
+    uint32_t i[1];
+    s.folded_indices<1>(d, i);
+    float a, b;
+    s.point<false>(dim, i[0], a, b);
+    return a;
+  }
+  static __device__ __noinline__ float2 draw_2(PathSamplerDev s, uint32_t dim) {
+    const uint32_t d[1] = {dim};
+    uint32_t i[1];
+    s.folded_indices<1>(d, i);
+    float2 r;
+    s.point<true>(dim, i[0], r.x, r.y);
+    return r;
+  }
+  // a 2D and a 1D draw (z) of one vertex together: the digit's share of the work
+  // once, and two independent chains for the scheduler
+  static __device__ __noinline__ float3 draw_21(PathSamplerDev s, uint32_t dim2, uint32_t dim1) {
+    const uint32_t d[2] = {dim2, dim1};
+    uint32_t i[2];
+    s.folded_indices<2>(d, i);
+    float3 r;
+    float unused;
+    s.point<true>(dim2, i[0], r.x, r.y);
+    s.point<false>(dim1, i[1], r.z, unused);
+    return r;
+  }
+  // 1D draws of four consecutive dimensions
+  static __device__ __noinline__ float4 draw_1111(PathSamplerDev s, uint32_t dim) {
+    const uint32_t d[4] = {dim, dim + 1u, dim + 2u, dim + 3u};
+    uint32_t i[4];
+    s.folded_indices<4>(d, i);
+    float4 r;
+    float unused;
+    s.point<false>(d[0], i[0], r.x, unused);
+    s.point<false>(d[1], i[1], r.y, unused);
+    s.point<false>(d[2], i[2], r.z, unused);
+    s.point<false>(d[3], i[3], r.w, unused);
+    return r;
+  }
+  __device__ __forceinline__ float4 sample_1d4(uint32_t first_dim) const { return draw_1111(*this, first_dim); }
+  __device__ __forceinline__ float sample_1d(uint32_t dim) const { return draw_1(*this, dim); }
   __device__ __forceinline__ void sample_2d(uint32_t dim, float& a, float& b) const {
-    float v[2];
-    sobol(dim, 2, v);
-    a = v[0];
-    b = v[1];
+    const float2 r = draw_2(*this, dim);
+    a = r.x;
+    b = r.y;
+  }
+  __device__ __forceinline__ void sample_2d_1d(uint32_t dim2, uint32_t dim1, float& a, float& b, float& c) const {
+    const float3 r = draw_21(*this, dim2, dim1);
+    a = r.x;
+    b = r.y;
+    c = r.z;
   }
   __device__ __forceinline__ uint32_t aux_rng_seed(uint32_t dim) const {
-    const uint64_t si = sample_index(dim);
+    uint64_t si;
+    if (narrow()) {
+      const uint32_t d[1] = {dim};
+      uint32_t i[1];
+      sample_index32<1>((uint32_t)morton, log2_spp, n_base4_digits, d, i);
+      si = i[0];
+    } else {
+      si = sample_index(dim);
+    }
     const uint64_t bits = mix_bits(si ^ ((uint64_t)dim << 32) ^ (uint64_t)seed);
     return pcg_hash((uint32_t)bits ^ (uint32_t)(bits >> 32));
   }

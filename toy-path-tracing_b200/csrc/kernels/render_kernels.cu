@@ -147,13 +147,9 @@ __global__ void __launch_bounds__(kRenderBlock, TPT_MK_MINB) render_mis_kernel(c
         done = true;  // pure emitter: no NEE, and sample() is None
       } else {
         if (alpha && P.integrator == kIntegMis) aux = aux_from_seed(ps, (int)depth);
-        float us0, us1;
-        ps.sample_2d(vertex_dim(depth, kOffSurface), us0, us1);
-        const float u_tree = ps.sample_1d(vertex_dim(depth, kOffTree));
-        const float u_cat = LIGHTS && S.d.num_cat > 1 ? ps.sample_1d(vertex_dim(depth, kOffCategory)) : 0.0f;
         DirectPrep dp;
         const bool nee = P.integrator != kIntegPt &&  // PT: BSDF sampling only
-                         prepare_direct<LIGHTS>(S, m, v, u_cat, u_tree, us0, us1, dp, P.integrator == kIntegNee);
+                         prepare_direct<LIGHTS>(S, m, v, ps, depth, dp, P.integrator == kIntegNee);
         if (nee) {
           contrib = beta * dp.contrib;
           tgt_inst = dp.inst;

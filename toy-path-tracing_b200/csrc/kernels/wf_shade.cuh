@@ -115,14 +115,9 @@ __global__ void __launch_bounds__(kWfBlock, ADJ ? 1 : 2) wf_shade(const __grid_c
           nx_aux = aux_from_seed(ps, (int)d + 1);
         }
       }
-      float us0, us1;
-      ps.sample_2d(vertex_dim(d, kOffSurface), us0, us1);
-      const float u_tree = ps.sample_1d(vertex_dim(d, kOffTree));
-      // one light-sampler category takes any u: skip drawing it
-      const float u_cat = LIGHTS && S.d.num_cat > 1 ? ps.sample_1d(vertex_dim(d, kOffCategory)) : 0.0f;
       // (PT: BSDF sampling only)
       if (P.integrator != kIntegPt &&
-          prepare_direct<LIGHTS>(S, m, v, u_cat, u_tree, us0, us1, dp, P.integrator == kIntegNee)) {
+          prepare_direct<LIGHTS>(S, m, v, ps, d, dp, P.integrator == kIntegNee)) {
         dp.contrib = beta * dp.contrib;
         push_shadow = true;
       }
