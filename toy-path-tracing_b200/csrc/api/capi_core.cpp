@@ -419,7 +419,8 @@ tpt_status tpt_scene_upload(tpt_context* ctx, const tpt_scene_desc* desc, tpt_sc
   const int threads = host_threads(0);
 
   std::vector<DevNode> nodes;
-  std::vector<DevTri> tris;
+  std::vector<DevTriPair> tris;
+  uint64_t n_tris = 0;  // triangles in `tris`, two per record
   std::vector<uint32_t> mesh_node_base(desc->num_meshes), mesh_tri_base(desc->num_meshes),
       mesh_root(desc->num_meshes);
   std::vector<uint32_t> tri_counts(desc->num_meshes);
@@ -481,7 +482,7 @@ tpt_status tpt_scene_upload(tpt_context* ctx, const tpt_scene_desc* desc, tpt_sc
       return set_error(ctx, TPT_ERR_INVALID_ARG, "mesh " + std::to_string(m) + " QBVH invalid: " +
                                                      (qpn != ntri ? std::string("primitive count mismatch") : why));
     mesh_node_base[m] = (uint32_t)nodes.size();
-    mesh_tri_base[m] = (uint32_t)tris.size();
+    mesh_tri_base[m] = (uint32_t)n_tris;
     mesh_root[m] = qnn ? 0u : (kLeafFlag | ((uint32_t)qpn << 24));
     tri_counts[m] = (uint32_t)ntri;
     for (uint64_t i = 0; i < qnn; ++i) nodes.push_back(to_dev(qn[i]));
@@ -494,14 +495,15 @@ tpt_status tpt_scene_upload(tpt_context* ctx, const tpt_scene_desc* desc, tpt_sc
       float vx = b.x - a.x, vy = b.y - a.y, vz = b.z - a.z;
       float cx = uy * vz - vy * uz, cy = uz * vx - vz * ux, cz = ux * vy - vx * uy;
       float l2 = cx * cx + cy * cy + cz * cz;
-      DevTri d;
       uint32_t tb = t;
       float tf;
       std::memcpy(&tf, &tb, 4);
-      d.v0 = make_float4(a.x, a.y, a.z, tf);
-      d.v1 = make_float4(b.x, b.y, b.z, l2 == 0.0f ? 1.0f : 0.0f);
-      d.v2 = make_float4(c.x, c.y, c.z, 0.0f);
-      tris.push_back(d);
+      const uint32_t half = (uint32_t)(n_tris++ & 1u);
+      if (half == 0) tris.push_back(DevTriPair{});
+      DevTriPair& d = tris.back();
+      d.v01[half][0] = make_float4(a.x, a.y, a.z, tf);
+      d.v01[half][1] = make_float4(b.x, b.y, b.z, l2 == 0.0f ? 1.0f : 0.0f);
+      d.v2[half] = make_float4(c.x, c.y, c.z, 0.0f);
     }
   }
 

@@ -8,8 +8,10 @@
 //              owning structure: interior = node index from its node base,
 //              leaf = offset from its primitive base.  Empty lanes hold
 //              0x80000000 and are skipped without a box test.
-//  - tris:     per mesh, triangles in BLAS leaf order, 48 B each: v0.xyz +
-//              triangle index, v1.xyz + degenerate flag, v2.xyz + 0.
+//  - tris:     per mesh, triangles in BLAS leaf order, 48 B each (v0.xyz +
+//              triangle index, v1.xyz + degenerate flag, v2.xyz + 0), stored as
+//              96 B pairs so that a triangle's first two vertices are one
+//              aligned 32-byte load: the pair's (v0, v1), (v0, v1), v2, v2.
 //  - instances: 64 B each: world_to_local as 4 columns of 3 floats (glam
 //              transform_point3 order), BLAS node base, triangle base, root
 //              word and material.
@@ -36,6 +38,12 @@ struct __align__(16) DevTri {
   float4 v2;
 };
 
+struct __align__(32) DevTriPair {  // triangles 2k and 2k + 1 of the concatenated meshes
+  float4 v01[2][2];
+  float4 v2[2];
+};
+static_assert(sizeof(DevTriPair) == 96, "triangle pair record");
+
 struct __align__(16) DevInstance {
   float4 m0;  // c0.x c0.y c0.z c1.x
   float4 m1;  // c1.y c1.z c2.x c2.y
@@ -49,7 +57,7 @@ static_assert(sizeof(DevInstance) == 64, "instance record");
 
 struct DevGeometry {
   const DevNode* nodes;
-  const DevTri* tris;
+  const DevTriPair* tris;
   const DevInstance* instances;
   const uint32_t* tlas_prims;  // TLAS primitive_indices (instance ids)
   uint32_t tlas_node_base;

@@ -20,6 +20,14 @@
 //    is kept iff u < the material's opacity, in the candidates' test order.
 // The library is compiled with -fmad=false so that no multiply-add is fused
 // unless written as fmaf (the reference's `mul_add`).
+//
+// What bounds it is not DRAM (the tree is L2-resident) but the L1 data pipe and
+// then the issue slots: lanes of incoherent rays read different nodes, and a
+// lane's load takes one cycle of the SM's load pipe whether it is 16 or 32 bytes
+// wide (measured: 7 x 16 B = 6.9 cycles per node and lane, 3 x 32 + 16 B = 3.9).
+// Hence 32-byte loads: four per node instead of seven, two per triangle instead
+// of three.  For the issue slots: packed two-lane subtracts and multiplies,
+// three-input min/max, and a branch-free ranking of the children.
 #pragma once
 #include "dev_types.cuh"
 
@@ -31,32 +39,42 @@ __device__ __forceinline__ float safe_inv(float d) { return d == 0.0f ? __int_as
 struct RayPre {
   float ox, oy, oz;     // origin
   float ix, iy, iz;     // safe reciprocal direction
-  float dx, dy, dz;     // direction
   float sx, sy, sz;     // shear constants of the watertight test
-  int kx, ky, kz;       // axis permutation (kz = largest |d| component)
+  int kz;               // axis of the largest |d| component; x, y follow it cyclically
   bool exact;           // an infinite reciprocal lane: use select min/max
   bool no_tri;          // permuted d.z == 0: no triangle can be hit
 };
 
-__device__ __forceinline__ float pick3(float a, float b, float c, int k) { return k == 0 ? a : (k == 1 ? b : c); }
+// (kx, ky, kz) components, kx = kz + 1 and ky = kz + 2 modulo 3
+__device__ __forceinline__ void permute3(float x, float y, float z, int kz, float& px, float& py, float& pz) {
+  px = kz == 0 ? y : (kz == 1 ? z : x);
+  py = kz == 0 ? z : (kz == 1 ? x : y);
+  pz = kz == 0 ? x : (kz == 1 ? y : z);
+}
 
 __device__ __forceinline__ void ray_setup(RayPre& r, float ox, float oy, float oz, float dx, float dy, float dz) {
   r.ox = ox; r.oy = oy; r.oz = oz;
-  r.dx = dx; r.dy = dy; r.dz = dz;
   r.ix = safe_inv(dx); r.iy = safe_inv(dy); r.iz = safe_inv(dz);
   // NaN can only come from 0 * inf in (b - o) * inv, i.e. from a reciprocal
   // lane that is infinite (or zero, for an infinite direction component).
   r.exact = !(isfinite(r.ix) && isfinite(r.iy) && isfinite(r.iz) && r.ix != 0.0f && r.iy != 0.0f && r.iz != 0.0f);
   float ax = fabsf(dx), ay = fabsf(dy), az = fabsf(dz);
   int kz = (ax > ay) ? (ax > az ? 0 : 2) : (ay > az ? 1 : 2);  // math/mod.rs:148-156
-  int kx = kz + 1; if (kx == 3) kx = 0;
-  int ky = kx + 1; if (ky == 3) ky = 0;
-  r.kx = kx; r.ky = ky; r.kz = kz;
-  float pdx = pick3(dx, dy, dz, kx), pdy = pick3(dx, dy, dz, ky), pdz = pick3(dx, dy, dz, kz);
+  r.kz = kz;
+  float pdx, pdy, pdz;
+  permute3(dx, dy, dz, kz, pdx, pdy, pdz);
   r.no_tri = (pdz == 0.0f);
   r.sx = -pdx / pdz;
   r.sy = -pdy / pdz;
-  r.sz = 1.0f / pdz;
+  r.sz = kz == 0 ? r.ix : (kz == 1 ? r.iy : r.iz);  // 1 / pdz (a zero pdz hits no triangle)
+}
+
+// The part of ray_setup that box tests read: at the TLAS no triangle is tested.
+__device__ __forceinline__ void ray_setup_boxes(RayPre& r, float ox, float oy, float oz, float dx, float dy,
+                                                float dz) {
+  r.ox = ox; r.oy = oy; r.oz = oz;
+  r.ix = safe_inv(dx); r.iy = safe_inv(dy); r.iz = safe_inv(dz);
+  r.exact = !(isfinite(r.ix) && isfinite(r.iy) && isfinite(r.iz) && r.ix != 0.0f && r.iy != 0.0f && r.iz != 0.0f);
 }
 
 __device__ __forceinline__ float dop(float a, float b, float c, float d) {
@@ -71,15 +89,15 @@ __device__ __forceinline__ bool tri_test(const RayPre& r, float t_max, const Dev
                                          float& b1, float& b2) {
   // degenerate flag precomputed on the host with the reference's formula
   if (tri.v1.w != 0.0f || r.no_tri) return false;
-  float p0x = pick3(tri.v0.x, tri.v0.y, tri.v0.z, r.kx) - pick3(r.ox, r.oy, r.oz, r.kx);
-  float p0y = pick3(tri.v0.x, tri.v0.y, tri.v0.z, r.ky) - pick3(r.ox, r.oy, r.oz, r.ky);
-  float p0z = pick3(tri.v0.x, tri.v0.y, tri.v0.z, r.kz) - pick3(r.ox, r.oy, r.oz, r.kz);
-  float p1x = pick3(tri.v1.x, tri.v1.y, tri.v1.z, r.kx) - pick3(r.ox, r.oy, r.oz, r.kx);
-  float p1y = pick3(tri.v1.x, tri.v1.y, tri.v1.z, r.ky) - pick3(r.ox, r.oy, r.oz, r.ky);
-  float p1z = pick3(tri.v1.x, tri.v1.y, tri.v1.z, r.kz) - pick3(r.ox, r.oy, r.oz, r.kz);
-  float p2x = pick3(tri.v2.x, tri.v2.y, tri.v2.z, r.kx) - pick3(r.ox, r.oy, r.oz, r.kx);
-  float p2y = pick3(tri.v2.x, tri.v2.y, tri.v2.z, r.ky) - pick3(r.ox, r.oy, r.oz, r.ky);
-  float p2z = pick3(tri.v2.x, tri.v2.y, tri.v2.z, r.kz) - pick3(r.ox, r.oy, r.oz, r.kz);
+  // permute, then translate: each component's subtraction as the reference's
+  float ox, oy, oz, p0x, p0y, p0z, p1x, p1y, p1z, p2x, p2y, p2z;
+  permute3(r.ox, r.oy, r.oz, r.kz, ox, oy, oz);
+  permute3(tri.v0.x, tri.v0.y, tri.v0.z, r.kz, p0x, p0y, p0z);
+  permute3(tri.v1.x, tri.v1.y, tri.v1.z, r.kz, p1x, p1y, p1z);
+  permute3(tri.v2.x, tri.v2.y, tri.v2.z, r.kz, p2x, p2y, p2z);
+  p0x -= ox; p0y -= oy; p0z -= oz;
+  p1x -= ox; p1y -= oy; p1z -= oz;
+  p2x -= ox; p2y -= oy; p2z -= oz;
   p0x = p0x + r.sx * p0z; p0y = p0y + r.sy * p0z;
   p1x = p1x + r.sx * p1z; p1y = p1y + r.sy * p1z;
   p2x = p2x + r.sx * p2z; p2y = p2y + r.sy * p2z;
@@ -119,38 +137,96 @@ __device__ __forceinline__ bool tri_test(const RayPre& r, float t_max, const Dev
   return true;
 }
 
+// One 32-byte read-only load (32-byte aligned).
+__device__ __forceinline__ void ldg32(const void* p, float (&v)[8]) {
+  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+      : "l"(p));
+}
+__device__ __forceinline__ float min3f(float a, float b, float c) {
+  float r;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ float max3f(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+// (b[k] - o) * i for the four lanes of a plane vector, two lanes per
+// instruction; each rounds as the scalar subtract and multiply do (b - o is
+// b + (-o)).
+__device__ __forceinline__ void slab4(const float* b, float o, float i, float (&t)[4]) {
+  asm("{\n\t"
+      ".reg .b64 p, q, n, m;\n\t"
+      "mov.b64 p, {%4, %5};\n\t"
+      "mov.b64 q, {%6, %7};\n\t"
+      "mov.b64 n, {%8, %8};\n\t"
+      "mov.b64 m, {%9, %9};\n\t"
+      "add.rn.f32x2 p, p, n;\n\t"
+      "add.rn.f32x2 q, q, n;\n\t"
+      "mul.rn.f32x2 p, p, m;\n\t"
+      "mul.rn.f32x2 q, q, m;\n\t"
+      "mov.b64 {%0, %1}, p;\n\t"
+      "mov.b64 {%2, %3}, q;\n\t"
+      "}"
+      : "=f"(t[0]), "=f"(t[1]), "=f"(t[2]), "=f"(t[3])
+      : "f"(b[0]), "f"(b[1]), "f"(b[2]), "f"(b[3]), "f"(-o), "f"(i));
+}
+
 // Slab test of one 4-wide node: returns the lane hit mask, lane entry
 // distances in tmin[], child words in ch[].
 __device__ __forceinline__ uint32_t box4(const DevNode* __restrict__ n, const RayPre& r, float t_max, float tmin[4],
                                          uint32_t ch[4]) {
-  const float4 lx = __ldg(&n->lo_x), ly = __ldg(&n->lo_y), lz = __ldg(&n->lo_z);
-  const float4 hx = __ldg(&n->hi_x), hy = __ldg(&n->hi_y), hz = __ldg(&n->hi_z);
+  float q0[8], q1[8], q2[8];  // lo_x lo_y | lo_z hi_x | hi_y hi_z
+  ldg32(&n->lo_x, q0);
+  ldg32(&n->lo_z, q1);
+  ldg32(&n->hi_y, q2);
   const uint4 c = __ldg(&n->child);
-  const float lox[4] = {lx.x, lx.y, lx.z, lx.w}, loy[4] = {ly.x, ly.y, ly.z, ly.w}, loz[4] = {lz.x, lz.y, lz.z, lz.w};
-  const float hix[4] = {hx.x, hx.y, hx.z, hx.w}, hiy[4] = {hy.x, hy.y, hy.z, hy.w}, hiz[4] = {hz.x, hz.y, hz.z, hz.w};
   ch[0] = c.x; ch[1] = c.y; ch[2] = c.z; ch[3] = c.w;
+  float t1x[4], t1y[4], t1z[4], t2x[4], t2y[4], t2z[4];
+  slab4(q0, r.ox, r.ix, t1x);
+  slab4(q0 + 4, r.oy, r.iy, t1y);
+  slab4(q1, r.oz, r.iz, t1z);
+  slab4(q1 + 4, r.ox, r.ix, t2x);
+  slab4(q2, r.oy, r.iy, t2y);
+  slab4(q2 + 4, r.oz, r.iz, t2z);
   uint32_t mask = 0;
+  if (!r.exact) {
 #pragma unroll
-  for (int s = 0; s < 4; ++s) {
-    float t1x = (lox[s] - r.ox) * r.ix, t2x = (hix[s] - r.ox) * r.ix;
-    float t1y = (loy[s] - r.oy) * r.iy, t2y = (hiy[s] - r.oy) * r.iy;
-    float t1z = (loz[s] - r.oz) * r.iz, t2z = (hiz[s] - r.oz) * r.iz;
-    float a, b;
-    if (r.exact) {
-      float mnx = t1x < t2x ? t1x : t2x, mxx = t1x > t2x ? t1x : t2x;
-      float mny = t1y < t2y ? t1y : t2y, mxy = t1y > t2y ? t1y : t2y;
-      float mnz = t1z < t2z ? t1z : t2z, mxz = t1z > t2z ? t1z : t2z;
-      a = mnx > mny ? mnx : mny; a = a > mnz ? a : mnz; a = a > 0.0f ? a : 0.0f;
-      b = mxx < mxy ? mxx : mxy; b = b < mxz ? b : mxz; b = b < t_max ? b : t_max;
-    } else {
-      a = fmaxf(fmaxf(fmaxf(fminf(t1x, t2x), fminf(t1y, t2y)), fminf(t1z, t2z)), 0.0f);
-      b = fminf(fminf(fminf(fmaxf(t1x, t2x), fmaxf(t1y, t2y)), fmaxf(t1z, t2z)), t_max);
+    for (int s = 0; s < 4; ++s) {
+      const float a = fmaxf(max3f(fminf(t1x[s], t2x[s]), fminf(t1y[s], t2y[s]), fminf(t1z[s], t2z[s])), 0.0f);
+      const float b = fminf(min3f(fmaxf(t1x[s], t2x[s]), fmaxf(t1y[s], t2y[s]), fmaxf(t1z[s], t2z[s])), t_max);
+      tmin[s] = a;
+      // lanes whose child word decodes to Empty (leaf bit, zero count) never count
+      if (a <= b && (ch[s] >> 24) != 0x80u) mask |= 1u << s;
     }
-    tmin[s] = a;
-    // lanes whose child word decodes to Empty (leaf bit, zero count) never count
-    if (a <= b && (ch[s] >> 24) != 0x80u) mask |= 1u << s;
+  } else {
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      const float mnx = t1x[s] < t2x[s] ? t1x[s] : t2x[s], mxx = t1x[s] > t2x[s] ? t1x[s] : t2x[s];
+      const float mny = t1y[s] < t2y[s] ? t1y[s] : t2y[s], mxy = t1y[s] > t2y[s] ? t1y[s] : t2y[s];
+      const float mnz = t1z[s] < t2z[s] ? t1z[s] : t2z[s], mxz = t1z[s] > t2z[s] ? t1z[s] : t2z[s];
+      float a = mnx > mny ? mnx : mny; a = a > mnz ? a : mnz; a = a > 0.0f ? a : 0.0f;
+      float b = mxx < mxy ? mxx : mxy; b = b < mxz ? b : mxz; b = b < t_max ? b : t_max;
+      tmin[s] = a;
+      if (a <= b && (ch[s] >> 24) != 0x80u) mask |= 1u << s;
+    }
   }
   return mask;
+}
+
+// Triangle g (index over all meshes) of the paired records: two loads, of 32 and
+// 16 bytes.
+__device__ __forceinline__ DevTri load_tri(const DevTriPair* __restrict__ tris, uint32_t g) {
+  const DevTriPair* p = tris + (g >> 1);
+  float q[8];
+  ldg32(&p->v01[g & 1u][0], q);
+  DevTri t;
+  t.v0 = make_float4(q[0], q[1], q[2], q[3]);
+  t.v1 = make_float4(q[4], q[5], q[6], q[7]);
+  t.v2 = __ldg(&p->v2[g & 1u]);
+  return t;
 }
 
 struct TraceResult {
@@ -166,17 +242,19 @@ struct TraceCounters {
 };
 
 // Per-thread traversal stack: the first SH entries live in shared memory
-// (entry k of thread i at base[k * blockDim.x], bank-conflict free), deeper
-// entries in a local-memory spill area.  Total depth kStackDepth (qbvh.rs:609).
-template <int SH>
+// (entry k of thread i at base[k * STRIDE], bank-conflict free; STRIDE is the
+// block size), deeper entries in a local-memory spill area.  Total depth
+// kStackDepth (qbvh.rs:609).
+template <int SH, int STRIDE>
 struct SplitStack {
+  static constexpr int kShared = SH, kStride = STRIDE;
   uint32_t* sh;
   uint32_t spill[kStackDepth - SH];
   __device__ __forceinline__ void set(int k, uint32_t v) {
-    if (k < SH) sh[k * blockDim.x] = v;
+    if (k < SH) sh[k * STRIDE] = v;
     else spill[k - SH] = v;
   }
-  __device__ __forceinline__ uint32_t get(int k) const { return k < SH ? sh[k * blockDim.x] : spill[k - SH]; }
+  __device__ __forceinline__ uint32_t get(int k) const { return k < SH ? sh[k * STRIDE] : spill[k - SH]; }
 };
 
 // Stack entries: interior node (bit 31 clear), BLAS/TLAS leaf (bit 31, count
@@ -190,15 +268,22 @@ struct TravState {
   float wox, woy, woz, wdx, wdy, wdz;  // world-space ray
   RayPre r;                            // ray of the current level (world at the TLAS, instance space in a BLAS)
   float closest;                       // running t_max
-  TraceResult res;
+  TraceResult res;                     // all but t, which hit_distance() gives
   uint32_t next;
   int sp, floor_sp;
   bool in_blas;
-  bool alpha_on;                       // an AuxRng state was given and the scene has alpha tests
-  uint32_t node_base, tri_base, inst_id;
+  uint32_t node_base;                  // first node of the current level (TLAS or BLAS)
+  uint32_t tri_base, inst_id;
+  // ALPHA instantiations only
+  bool alpha_on;                       // the scene has alpha tests
   float alpha;                         // the current instance's opacity (1: no test)
   uint32_t aux;                        // AuxRng state
 };
+
+// The hit's distance (+inf: no hit): the running t_max of the last accepted hit.
+__device__ __forceinline__ float hit_distance(const TravState& s) {
+  return s.res.tri >= 0 ? s.closest : __int_as_float(0x7f800000);
+}
 
 // AuxRng::next_f32 (aux_rng.rs:21-28)
 __device__ __forceinline__ float aux_next_f32(uint32_t& state) {
@@ -212,9 +297,10 @@ __device__ __forceinline__ float aux_next_f32(uint32_t& state) {
 
 // Enter instance `id`'s BLAS with the ray transformed by world_to_local
 // (glam Mat4::transform_point3 / transform_vector3 order), scene/mod.rs:357.
+template <bool ALPHA>
 __device__ __forceinline__ void enter_instance(const DevGeometry& G, TravState& s, uint32_t id) {
   s.inst_id = id;
-  s.alpha = s.alpha_on ? __ldg(G.inst_alpha + id) : 1.0f;
+  if (ALPHA) s.alpha = s.alpha_on ? __ldg(G.inst_alpha + id) : 1.0f;
   const DevInstance* I = G.instances + id;
   const float4 m0 = __ldg(&I->m0), m1 = __ldg(&I->m1), m2 = __ldg(&I->m2);
   const uint4 meta = __ldg(reinterpret_cast<const uint4*>(&I->node_base));
@@ -235,7 +321,7 @@ __device__ __forceinline__ void enter_instance(const DevGeometry& G, TravState& 
 }
 
 template <class Stack>
-__device__ __forceinline__ void trav_pop(TravState& s, Stack& st) {
+__device__ __forceinline__ void trav_pop(const DevGeometry& G, TravState& s, Stack& st) {
   if (s.sp == 0) {
     s.next = kNone;
     return;
@@ -243,35 +329,40 @@ __device__ __forceinline__ void trav_pop(TravState& s, Stack& st) {
   if (s.in_blas && s.sp == s.floor_sp) {
     // the instance's BLAS is done: back to the TLAS with the world ray
     s.in_blas = false;
-    ray_setup(s.r, s.wox, s.woy, s.woz, s.wdx, s.wdy, s.wdz);
+    s.node_base = G.tlas_node_base;
+    ray_setup_boxes(s.r, s.wox, s.woy, s.woz, s.wdx, s.wdy, s.wdz);
   }
   s.next = st.get(--s.sp);
 }
 
-// aux: the ray's AuxRng state (NULL: no alpha tests), advanced by the draws
+// ALPHA: the caller has AuxRng states (aux: the ray's, NULL = none), which the
+// alpha tests of the scene's materials advance; without, no alpha test is made.
+template <bool ALPHA>
 __device__ __forceinline__ void trav_init(const DevGeometry& G, TravState& s, float ox, float oy, float oz, float dx,
-                                          float dy, float dz, float t_max, const uint32_t* aux = nullptr) {
-  s.alpha_on = aux != nullptr && G.inst_alpha != nullptr;
-  s.aux = aux ? *aux : 0u;
-  s.alpha = 1.0f;
+                                          float dy, float dz, float t_max, const uint32_t* aux) {
+  if (ALPHA) {
+    s.alpha_on = aux != nullptr && G.inst_alpha != nullptr;
+    s.aux = aux ? *aux : 0u;
+    s.alpha = 1.0f;
+  }
   s.wox = ox; s.woy = oy; s.woz = oz; s.wdx = dx; s.wdy = dy; s.wdz = dz;
   s.closest = t_max;
-  s.res.t = __int_as_float(0x7f800000);
   s.res.tri = -1;
   s.res.inst = -1;
   s.res.b0 = s.res.b1 = s.res.b2 = 0.0f;
   s.in_blas = false;
   s.floor_sp = 0;
   s.sp = 0;
-  s.node_base = s.tri_base = s.inst_id = 0;
+  s.node_base = G.tlas_node_base;
+  s.tri_base = s.inst_id = 0;
   s.next = kNone;
   if (G.num_instances == 0) return;
   const uint32_t root = G.tlas_root_word;
   if ((root & kLeafBit) && ((root >> 24) & 0x7Fu) == 1u) {
     // TLAS is a single-instance root leaf (qbvh.rs:615-620): go straight to it
-    enter_instance(G, s, __ldg(G.tlas_prims + (root & 0xFFFFFFu)));
+    enter_instance<ALPHA>(G, s, __ldg(G.tlas_prims + (root & 0xFFFFFFu)));
   } else {
-    ray_setup(s.r, ox, oy, oz, dx, dy, dz);
+    ray_setup_boxes(s.r, ox, oy, oz, dx, dy, dz);
     s.next = root;
   }
 }
@@ -280,89 +371,79 @@ __device__ __forceinline__ void trav_init(const DevGeometry& G, TravState& s, fl
 // top, as interiors far-to-near then leaves near-to-far (qbvh.rs:640-671: leaves
 // are handled far-to-near at once, the nearest interior is popped first); the
 // would-be top becomes `next`, the rest go to the stack.
+//
+// A child's key orders the hit children as they will be popped: leaves first,
+// far to near (the complemented distance, negative), then interiors near to
+// far (the distance's bits).  On equal distances the lower lane is the nearer
+// (stable order): it comes first among interiors and last among leaves, which
+// the +1 of an interior's right-hand key expresses.  Ranks from the six
+// comparisons place every child without branches, so the lanes of a warp stay
+// together: 13.8 instead of 10.7 active lanes per instruction and 17.0 instead
+// of 23.4 warp instructions per node test on incoherent rays.
 template <bool STATS, class Stack>
 __device__ __forceinline__ void node_step(const DevGeometry& G, TravState& s, Stack& st, TraceCounters& cnt,
                                           uint32_t* err) {
-  const DevNode* n = G.nodes + (s.in_blas ? s.node_base : G.tlas_node_base) + s.next;
+  const DevNode* n = G.nodes + s.node_base + s.next;
   if (STATS) cnt.nodes++;
   float tmin[4];
   uint32_t ch[4];
   const uint32_t mask = box4(n, s.r, s.closest, tmin, ch);
   const int nh = __popc(mask);
   if (nh == 0) {
-    trav_pop(s, st);
+    trav_pop(G, s, st);
     return;
   }
-  if (nh == 1) {
-    s.next = (mask & 1u) ? ch[0] : (mask & 2u) ? ch[1] : (mask & 4u) ? ch[2] : ch[3];
-    return;
-  }
-  if (s.sp + nh - 1 > kStackDepth) {
-    atomicOr(err, kDevErrStackOverflow);
-    s.sp = 0;
-    s.next = kNone;
-    return;
-  }
-  // before[i][j]: lane i precedes lane j in the stable ascending order by tmin
-  bool v[4], leaf[4];
+  int key[4], right[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    v[i] = (mask >> i) & 1u;
-    leaf[i] = (ch[i] & kLeafBit) != 0;
+    const int leaf = (int)ch[i] >> 31;  // all ones for a leaf
+    const int k = (__float_as_int(tmin[i]) & 0x7fffffff) ^ leaf;
+    key[i] = (mask >> i) & 1u ? k : 0x7ffffffe;  // not hit: behind every hit
+    right[i] = key[i] + 1 + leaf;
   }
-  bool pre[4][4];
+  const bool c01 = key[0] < right[1], c02 = key[0] < right[2], c03 = key[0] < right[3];
+  const bool c12 = key[1] < right[2], c13 = key[1] < right[3], c23 = key[2] < right[3];
+  const int rank[4] = {3 - c01 - c02 - c03, 2 + c01 - c12 - c13, 1 + c02 + c12 - c23, 0 + c03 + c13 + c23};
+  const int top = s.sp + nh - 1;  // entries on the stack afterwards
 #pragma unroll
   for (int i = 0; i < 4; ++i)
+    if (rank[i] == 0) s.next = ch[i];
+  if (top <= Stack::kShared) {
+    uint32_t* base = st.sh + top * Stack::kStride;
 #pragma unroll
-    for (int j = i + 1; j < 4; ++j) {
-      pre[i][j] = tmin[i] <= tmin[j];
-      pre[j][i] = !pre[i][j];
+    for (int i = 0; i < 4; ++i)
+      if (rank[i] > 0 && rank[i] < nh) base[-rank[i] * Stack::kStride] = ch[i];
+  } else {
+    if (top > kStackDepth) {
+      atomicOr(err, kDevErrStackOverflow);
+      s.sp = 0;
+      s.next = kNone;
+      return;
     }
-  int n_int = 0;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) n_int += (v[i] && !leaf[i]) ? 1 : 0;
-  const int top = nh - 1;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    if (!v[i]) continue;
-    int pos = 0;
-    if (!leaf[i]) {
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (j != i && v[j] && !leaf[j] && pre[i][j]) ++pos;  // interiors farther than i
-    } else {
-      pos = n_int;
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (j != i && v[j] && leaf[j] && pre[j][i]) ++pos;  // leaves nearer than i
-    }
-    if (pos == top) s.next = ch[i];
-    else st.set(s.sp + pos, ch[i]);
+    for (int i = 0; i < 4; ++i)
+      if (rank[i] > 0 && rank[i] < nh) st.set(top - rank[i], ch[i]);
   }
-  s.sp += nh - 1;
+  s.sp = top;
 }
 
 // Processes the leaf, TLAS leaf or instance marker in `next`.
-template <int MODE, bool STATS, class Stack>
+template <int MODE, bool STATS, bool ALPHA, class Stack>
 __device__ __forceinline__ void leaf_step(const DevGeometry& G, TravState& s, Stack& st, TraceCounters& cnt,
                                           uint32_t* err) {
   const uint32_t w = s.next;
   const uint32_t count = (w >> 24) & 0x7Fu, off = w & 0xFFFFFFu;
   if (s.in_blas) {
     // BLAS leaf: triangles in leaf order, t_max shrinking on each hit
-    const DevTri* T = G.tris + s.tri_base + off;
-    for (uint32_t j = 0; j < count; ++j) {
-      DevTri tri;
-      tri.v0 = __ldg(&T[j].v0);
-      tri.v1 = __ldg(&T[j].v1);
-      tri.v2 = __ldg(&T[j].v2);
+    uint32_t g = s.tri_base + off;
+    for (const uint32_t end = g + count; g != end; ++g) {
+      const DevTri tri = load_tri(G.tris, g);
       if (STATS) cnt.tris++;
       float t, b0, b1, b2;
       if (tri_test(s.r, s.closest, tri, t, b0, b1, b2)) {
         // any_hit of an alpha-tested material: keep the hit iff u < opacity
-        if (s.alpha < 1.0f && !(aux_next_f32(s.aux) < s.alpha)) continue;
+        if (ALPHA && s.alpha < 1.0f && !(aux_next_f32(s.aux) < s.alpha)) continue;
         s.closest = t;
-        s.res.t = t;
         s.res.tri = __float_as_int(tri.v0.w);
         s.res.inst = (int32_t)s.inst_id;
         s.res.b0 = b0; s.res.b1 = b1; s.res.b2 = b2;
@@ -373,9 +454,9 @@ __device__ __forceinline__ void leaf_step(const DevGeometry& G, TravState& s, St
         }
       }
     }
-    trav_pop(s, st);
+    trav_pop(G, s, st);
   } else if (count == 0) {
-    enter_instance(G, s, off);
+    enter_instance<ALPHA>(G, s, off);
   } else {
     // TLAS leaf: its instances in order; the first is entered now
     if (s.sp + (int)count > kStackDepth) {
@@ -385,7 +466,7 @@ __device__ __forceinline__ void leaf_step(const DevGeometry& G, TravState& s, St
       return;
     }
     for (int j = (int)count - 1; j >= 1; --j) st.set(s.sp++, kLeafBit | __ldg(G.tlas_prims + off + j));
-    enter_instance(G, s, __ldg(G.tlas_prims + off));
+    enter_instance<ALPHA>(G, s, __ldg(G.tlas_prims + off));
   }
 }
 
@@ -395,13 +476,14 @@ __device__ __forceinline__ void trace_ray(const DevGeometry& G, Stack& st, float
                                           float dy, float dz, float t_max, TraceResult& res, TraceCounters& cnt,
                                           uint32_t* err, uint32_t* aux = nullptr) {
   TravState s;
-  trav_init(G, s, ox, oy, oz, dx, dy, dz, t_max, aux);
+  trav_init<true>(G, s, ox, oy, oz, dx, dy, dz, t_max, aux);
   if (STATS) { cnt.nodes = 0; cnt.tris = 0; }
   while (s.next != kNone) {
     if (!(s.next & kLeafBit)) node_step<STATS>(G, s, st, cnt, err);
-    else leaf_step<MODE, STATS>(G, s, st, cnt, err);
+    else leaf_step<MODE, STATS, true>(G, s, st, cnt, err);
   }
   res = s.res;
+  res.t = hit_distance(s);
   if (aux) *aux = s.aux;
 }
 
@@ -415,17 +497,18 @@ __device__ __forceinline__ void trace_ray_ww(const DevGeometry& G, Stack& st, un
                                              uint32_t* err, uint32_t* aux = nullptr) {
   TravState s;
   TraceCounters c;
-  trav_init(G, s, ox, oy, oz, dx, dy, dz, t_max, aux);
+  trav_init<true>(G, s, ox, oy, oz, dx, dy, dz, t_max, aux);
   for (;;) {
     for (;;) {
       const bool want = !(s.next & kLeafBit);
       if (!__any_sync(act, want)) break;
       if (want) node_step<false>(G, s, st, c, err);
     }
-    if (s.next != kNone) leaf_step<MODE, false>(G, s, st, c, err);
+    if (s.next != kNone) leaf_step<MODE, false, true>(G, s, st, c, err);
     if (!__any_sync(act, s.next != kNone)) break;
   }
   res = s.res;
+  res.t = hit_distance(s);
   if (aux) *aux = s.aux;
 }
 

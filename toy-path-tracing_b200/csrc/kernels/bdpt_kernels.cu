@@ -14,7 +14,7 @@ __global__ void __launch_bounds__(kBdptBlock) render_bdpt_kernel(const __grid_co
                                                                  float* __restrict__ samples, uint64_t first_path,
                                                                  uint64_t n_paths, uint32_t* err) {
   __shared__ uint32_t stack_sh[kBdptShStack * kBdptBlock];
-  SplitStack<kBdptShStack> st;
+  SplitStack<kBdptShStack, kBdptBlock> st;
   st.sh = stack_sh + threadIdx.x;
   // warp-uniform loop: the lanes of a warp take consecutive samples together
   // (trace_bdpt is warp-synchronous); lanes past the end carry no sample

@@ -43,7 +43,7 @@ __global__ void __launch_bounds__(kRenderBlock, TPT_MK_MINB) render_mis_kernel(c
                                                                   unsigned long long* __restrict__ counter,
                                                                   uint32_t* err) {
   __shared__ uint32_t stack_sh[kRenderShStack * kRenderBlock];
-  SplitStack<kRenderShStack> st;
+  SplitStack<kRenderShStack, kRenderBlock> st;
   st.sh = stack_sh + threadIdx.x;
   const unsigned lane = threadIdx.x & 31u;
   int64_t k = -1;  // path (relative to first_path); -1: needs one, -2: none left

@@ -7,8 +7,10 @@
 // tested together, then finished lanes get new rays from a global counter by
 // one warp-aggregated atomic.  Batching keeps the warp on one code path at a
 // time without changing any ray's own visit order.
-// Traversal stacks: 32 entries per thread in shared memory, spilling to local
-// memory beyond that (total depth 128, as the reference).
+// Traversal stacks: kShStack entries per thread in shared memory, spilling to
+// local memory beyond that (total depth 128, as the reference).  Twelve cover
+// nearly every ray of a 1M-triangle tree, and each entry less leaves more of the
+// SM's memory to the L1 cache.
 // Counting (STATS): per-ray node and triangle test counts into node_tests /
 // tri_tests when given, and, when `totals` is given, the launch's sums added
 // to totals[0..3] = rays, 4-wide node tests, triangle tests, hits (one atomic
@@ -22,16 +24,22 @@
 namespace tpt {
 
 constexpr int kBlock = 128;
-constexpr int kShStack = 32;
-#ifndef TPT_TRAV_MINB
-#define TPT_TRAV_MINB 8
-#endif
-#ifndef TPT_REFILL_MIN
-#define TPT_REFILL_MIN 12  // finished lanes that end the node phase early for a refill
-#endif
+constexpr int kShStack = 12;
+// Blocks per SM: 7 leave 72 registers, which the kernel fits without spilling
+// (8 blocks spill some 100 bytes a thread).
+constexpr int kMinBlocks = 7;
+// Finished lanes that end the node phase early for a refill, and the lanes still
+// at interior nodes below which those waiting at a leaf go first: without the
+// second rule the last ray of a warp to reach a leaf holds up the other 31.
+// Measured (2^24 incoherent rays on 1M triangles / 2^22 rays on the 2.1M-
+// triangle instanced scene / 2^22 rays in the Cornell box, ms): 16-byte loads
+// and branches 8.15 / 5.70 / 3.11; this kernel with kNodeMin 0 5.94 / 4.61 / 2.44,
+// 8 5.88 / 3.66 / 2.10, 11 5.92 / 3.69 / 2.01.  kRefillMin 8 or 16: 4 % and 1 % slower.
+constexpr int kRefillMin = 12;
+constexpr int kNodeMin = 8;
 
-template <int MODE, bool STATS, bool BARY, bool BATCH>
-__global__ void __launch_bounds__(kBlock, TPT_TRAV_MINB)
+template <int MODE, bool STATS, bool BARY, bool BATCH, bool ALPHA>
+__global__ void __launch_bounds__(kBlock, kMinBlocks)
     traverse_kernel(DevGeometry geo, const float* __restrict__ rays, uint64_t rs, uint64_t n, uint64_t bs,
                     int32_t* __restrict__ prim, float* __restrict__ tout, int32_t* __restrict__ inst,
                     float* __restrict__ bary, uint32_t* __restrict__ node_tests, uint32_t* __restrict__ tri_tests,
@@ -43,7 +51,7 @@ __global__ void __launch_bounds__(kBlock, TPT_TRAV_MINB)
   DevGeometry lane_geo;  // BATCH: the scene of this lane's ray
   const DevGeometry& G = BATCH ? lane_geo : geo;
   __shared__ uint32_t stack_sh[kShStack * kBlock];
-  SplitStack<kShStack> st;
+  SplitStack<kShStack, kBlock> st;
   st.sh = stack_sh + threadIdx.x;
   const unsigned lane = threadIdx.x & 31u;
   const unsigned lt_mask = (1u << lane) - 1u;
@@ -72,7 +80,7 @@ __global__ void __launch_bounds__(kBlock, TPT_TRAV_MINB)
           const float dx = __ldcs(rays + 3 * rs + i), dy = __ldcs(rays + 4 * rs + i), dz = __ldcs(rays + 5 * rs + i);
           const float tmax = MODE == 0 ? __int_as_float(0x7f800000) : __ldcs(rays + 6 * rs + i);
           if (BATCH) lane_geo = jobs[__ldg(ray_job + i)].render.geo;
-          trav_init(G, s, ox, oy, oz, dx, dy, dz, tmax, aux ? aux + (aux_index ? aux_index[i] : i) : nullptr);
+          trav_init<ALPHA>(G, s, ox, oy, oz, dx, dy, dz, tmax, ALPHA ? aux + (aux_index ? aux_index[i] : i) : nullptr);
           if (STATS) { c.nodes = 0; c.tris = 0; }
         } else {
           ray = -2;
@@ -81,13 +89,18 @@ __global__ void __launch_bounds__(kBlock, TPT_TRAV_MINB)
     }
     if (__all_sync(0xffffffffu, ray == -2)) break;
     const bool active = ray >= 0;
-    // phase A: interior nodes until every active lane faces a leaf, or until
+    // phase A: interior nodes until every active lane faces a leaf, until
     // enough lanes have finished their ray to be worth a refill (lanes with no
-    // ray left do not count: they can never be refilled)
+    // ray left do not count: they can never be refilled), or until few lanes
+    // are left at interior nodes while others wait at a leaf
     for (;;) {
       const bool want = active && !(s.next & kLeafBit);
-      if (!__any_sync(0xffffffffu, want)) break;
-      if (__popc(__ballot_sync(0xffffffffu, active && s.next == kNone)) >= TPT_REFILL_MIN) break;
+      const unsigned wm = __ballot_sync(0xffffffffu, want);
+      if (!wm) break;
+      if (__popc(__ballot_sync(0xffffffffu, active && s.next == kNone)) >= kRefillMin) break;
+      if (__popc(wm) < kNodeMin &&
+          __any_sync(0xffffffffu, active && s.next != kNone && (s.next & kLeafBit)))
+        break;
       if (want) {
         node_step<STATS>(G, s, st, c, err);
         moved = true;
@@ -95,15 +108,15 @@ __global__ void __launch_bounds__(kBlock, TPT_TRAV_MINB)
     }
     // phase B: one leaf / instance entry per lane
     if (active && s.next != kNone && (s.next & kLeafBit)) {
-      leaf_step<MODE, STATS>(G, s, st, c, err);
+      leaf_step<MODE, STATS, ALPHA>(G, s, st, c, err);
       moved = true;
     }
     if (active && s.next == kNone) {
       moved = true;
       const uint64_t i = (uint64_t)ray;
       __stcs(prim + i, s.res.tri);
-      __stcs(tout + i, s.res.t);
-      if (aux) aux[aux_index ? aux_index[i] : i] = s.aux;
+      __stcs(tout + i, hit_distance(s));
+      if (ALPHA) aux[aux_index ? aux_index[i] : i] = s.aux;
       if (inst) __stcs(inst + i, s.res.inst);
       if (BARY) {
         __stcs(bary + i, s.res.b0);
@@ -149,7 +162,7 @@ __global__ void __launch_bounds__(kBlock, TPT_TRAV_MINB)
   }
 }
 
-template <int MODE, bool STATS, bool BARY, bool BATCH>
+template <int MODE, bool STATS, bool BARY, bool BATCH, bool ALPHA>
 static cudaError_t launch_t(const DevGeometry& geo, const float* rays, uint64_t rs, uint64_t n, uint64_t bs,
                             int32_t* prim, float* t, int32_t* inst, float* bary, uint32_t* nt, uint32_t* tt,
                             unsigned long long* counter, const uint32_t* n_dev, uint32_t* err, int num_sms,
@@ -159,7 +172,7 @@ static cudaError_t launch_t(const DevGeometry& geo, const float* rays, uint64_t 
   static int blocks_per_sm = 0;
   if (blocks_per_sm == 0) {
     cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &blocks_per_sm, traverse_kernel<MODE, STATS, BARY, BATCH>, kBlock, 0);
+        &blocks_per_sm, traverse_kernel<MODE, STATS, BARY, BATCH, ALPHA>, kBlock, 0);
     if (e != cudaSuccess || blocks_per_sm <= 0) blocks_per_sm = 4;
   }
   uint64_t blocks = (uint64_t)num_sms * blocks_per_sm;
@@ -167,7 +180,7 @@ static cudaError_t launch_t(const DevGeometry& geo, const float* rays, uint64_t 
   if (blocks > need) blocks = need;
   cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), s);
   if (e != cudaSuccess) return e;
-  traverse_kernel<MODE, STATS, BARY, BATCH><<<(unsigned)blocks, kBlock, 0, s>>>(
+  traverse_kernel<MODE, STATS, BARY, BATCH, ALPHA><<<(unsigned)blocks, kBlock, 0, s>>>(
       geo, rays, rs, n, bs, prim, t, inst, bary, nt, tt, counter, n_dev, err, jobs, ray_job, totals, aux, aux_index);
   return cudaGetLastError();
 }
@@ -180,23 +193,27 @@ cudaError_t launch_traverse_strided(const DevGeometry& geo, const float* rays, u
                                     const uint32_t* aux_index) {
   const bool stats = nt != nullptr || totals != nullptr;
   const bool b = bary != nullptr;
-#define TPT_L(M, S, B, J) \
-  launch_t<M, S, B, J>(geo, rays, rs, n, bs, prim, t, inst, bary, nt, tt, counter, n_dev, err, num_sms, s, jobs, \
-                       ray_job, totals, aux, aux_index)
+#define TPT_LA(M, S, B, J, A) \
+  launch_t<M, S, B, J, A>(geo, rays, rs, n, bs, prim, t, inst, bary, nt, tt, counter, n_dev, err, num_sms, s, jobs, \
+                          ray_job, totals, aux, aux_index)
+// alpha tests draw from AuxRng states, which closest-hit queries alone carry
+#define TPT_L(S, B, J) (aux ? TPT_LA(0, S, B, J, true) : TPT_LA(0, S, B, J, false))
   if (jobs) {  // batched wavefront: closest hit, with or without barycentrics
     if (mode != 0 || stats) return cudaErrorInvalidValue;
-    if (b) return TPT_L(0, false, true, true);
-    return TPT_L(0, false, false, true);
+    if (b) return TPT_L(false, true, true);
+    return TPT_L(false, false, true);
   }
   if (mode == 0) {
-    if (stats && b) return TPT_L(0, true, true, false);
-    if (stats) return TPT_L(0, true, false, false);
-    if (b) return TPT_L(0, false, true, false);
-    return TPT_L(0, false, false, false);
+    if (stats && b) return TPT_L(true, true, false);
+    if (stats) return TPT_L(true, false, false);
+    if (b) return TPT_L(false, true, false);
+    return TPT_L(false, false, false);
   }
-  if (stats) return TPT_L(1, true, false, false);
-  if (b) return TPT_L(1, false, true, false);
-  return TPT_L(1, false, false, false);
+  if (aux) return cudaErrorInvalidValue;
+  if (stats) return TPT_LA(1, true, false, false, false);
+  if (b) return TPT_LA(1, false, true, false, false);
+  return TPT_LA(1, false, false, false, false);
+#undef TPT_LA
 #undef TPT_L
 }
 
