@@ -459,7 +459,9 @@ tpt_status tpt_context_set_graphs(tpt_context* ctx, int enable);
  * Megakernel and batched renders are not counted.  NULL turns it off.  Results
  * do not depend on it. */
 tpt_status tpt_context_set_render_stats(tpt_context* ctx, uint64_t* d_counters);
-/* Threads per block of the wavefront shade stage: 128 or 256 (default). */
+/* Block size of the wavefront shade stage: 128 = blocks of 128 threads, 256
+ * (default) = the stage's full blocks (384 threads: warps of one block share
+ * their instruction fetches). */
 tpt_status tpt_context_set_shade_block(tpt_context* ctx, uint32_t threads);
 
 /* Renders each job into out_rgb[j] (host, width*height*3 floats, row-major,
@@ -512,7 +514,7 @@ typedef struct tpt_tune_result {
   uint32_t execution;          /* TPT_EXEC_WAVEFRONT or TPT_EXEC_MEGAKERNEL */
   uint32_t wavefront_capacity; /* path slots per chunk */
   uint32_t graphs;             /* 1: bounces replayed from captured graphs */
-  uint32_t shade_block;        /* threads per block of the wavefront shade stage */
+  uint32_t shade_block;        /* tpt_context_set_shade_block's setting: 128 or 256 (full blocks) */
   float ms;                    /* last-pilot time of the chosen settings */
   float ms_megakernel;         /* last-pilot time of the megakernel */
   float ms_wavefront_default;  /* last-pilot time of the wavefront at 2^24 slots, graphs, the context's block */

@@ -988,6 +988,16 @@ struct Sample {
   float lock;     // the wavelength this sample locks the path to (< 0: none)
 };
 
+// What sample_dir returns: no sample; a finished one (delta lobes and lobes that
+// are weighted on the spot); or a rough lobe's direction (out.wi, out.flags),
+// which finalize weighs.
+enum SampleStep : int { kNoSample = 0, kSampled = 1, kRough = 2 };
+__device__ __forceinline__ SampleStep rough_direction(V3 wi, uint32_t flags, Sample& out) {
+  out.wi = wi;
+  out.flags = flags;
+  return kRough;
+}
+
 // finalize_rough_sample_with_wavelength (open_pbr.rs:1997-2027).  `importance`
 // selects the transport mode of the evaluation; `want_rev` computes pdf_rev.
 __device__ __forceinline__ bool finalize(const OpbrVertex& s, V3 wi, uint32_t flags, bool importance, bool want_rev,
@@ -1090,8 +1100,8 @@ static __device__ __noinline__ bool sample_btdf_channels(const OpbrVertex& s, fl
 // the path's locked wavelength, at a wavelength drawn with ux[0] (smooth, front
 // face: the path locks to it), or over sampled camera channels (rough, front
 // face, unlocked).
-static __device__ __noinline__ bool sample_btdf(const OpbrVertex& s, float p_lobe, float u0, float u1, Sample& out,
-                                                bool importance, bool want_rev, const float* ux) {
+static __device__ __noinline__ SampleStep sample_btdf(const OpbrVertex& s, float p_lobe, float u0, float u1,
+                                                      Sample& out, bool importance, const float* ux) {
   const DevOpenPbr& m = *s.m;
   const V3 wo = s.wo;
   const V3 one = V3{1.0f, 1.0f, 1.0f};
@@ -1104,27 +1114,27 @@ static __device__ __noinline__ bool sample_btdf(const OpbrVertex& s, float p_lob
       out.wi = wi;
       out.pdf = p_lobe;
       out.flags = kFlagDelta | kFlagTransmission;
-      return true;
+      return kSampled;
     }
     V3 wm;
-    if (!sample_wm_bounded_vndf(wo, m.tw_ax, m.tw_ay, u0, u1, wm)) return false;
+    if (!sample_wm_bounded_vndf(wo, m.tw_ax, m.tw_ay, u0, u1, wm)) return kNoSample;
     const V3 wr = reflect_local(wo, wm);
-    if (wr.z <= 0.0f) return false;
+    if (wr.z <= 0.0f) return kNoSample;
     const V3 wi = V3{wr.x, wr.y, -wr.z};
     const V3 bw = weights_below(s, one).btdf;
     V3 fb, f_thin;
     float pb;
     btdf_eval_pdf(s, wi, importance, fb, pb, f_thin);
     const float pdf_total = p_lobe * pb;
-    if (pdf_total <= 0.0f) return false;
+    if (pdf_total <= 0.0f) return kNoSample;
     out.weight = bw * f_thin * fabsf(wi.z) / pdf_total;
     out.wi = wi;
     out.pdf = pdf_total;
     out.flags = kFlagGlossy | kFlagTransmission;
-    return true;  // pdf_rev = pdf(wi, wo) = 0: wi is below the surface
+    return kSampled;  // pdf_rev = pdf(wi, wo) = 0: wi is below the surface
   }
   if (m.flags & kOpbrDisp) {
-    if (camera_dispersion(s)) return sample_btdf_channels(s, p_lobe, u0, u1, ux, out, importance);
+    if (camera_dispersion(s)) return sample_btdf_channels(s, p_lobe, u0, u1, ux, out, importance) ? kSampled : kNoSample;
     if (s.lock >= 0.0f || s.face == 0u) {
       V3 basis = one;
       float eta_u;
@@ -1137,14 +1147,14 @@ static __device__ __noinline__ bool sample_btdf(const OpbrVertex& s, float p_lob
       const float eta_rel = s.face == 0u ? 1.0f / eta_u : eta_u;
       if (!rough) {
         V3 wi;
-        if (!refract_z(wo, eta_rel, wi)) return false;
+        if (!refract_z(wo, eta_rel, wi)) return kNoSample;
         const float fr = dielectric_fresnel_eta(m, s.face, fabsf(wo.z), eta_u, eta_u);
         const float scale = importance ? 1.0f : 1.0f / (eta_rel * eta_rel);
         out.weight = (weights_below(s, one).btdf * basis * (1.0f - fr) * scale) / p_lobe;
         out.wi = wi;
         out.pdf = p_lobe;
         out.flags = kFlagDelta | kFlagTransmission;
-        return true;
+        return kSampled;
       }
       // rough and locked: the locked eta's lobe weights, evaluated at the lock
       const TransMs tm = trans_ms_at(s, eta_u);
@@ -1157,29 +1167,29 @@ static __device__ __noinline__ bool sample_btdf(const OpbrVertex& s, float p_lob
       } else {
         const float uu = ss_p > 0.0f ? u0 / ss_p : 0.0f;
         V3 wm;
-        if (!sample_wm_vndf(wo, m.spec_ax, m.spec_ay, uu, u1, wm)) return false;
+        if (!sample_wm_vndf(wo, m.spec_ax, m.spec_ay, uu, u1, wm)) return kNoSample;
         const float co = dot(wo, wm);
-        if (co <= 0.0f) return false;
-        if (!refract_about(wo, wm, eta_rel, wi)) return false;
-        if (wi.z >= 0.0f) return false;
+        if (co <= 0.0f) return kNoSample;
+        if (!refract_about(wo, wm, eta_rel, wi)) return kNoSample;
+        if (wi.z >= 0.0f) return kNoSample;
         const float ci = dot(wi, wm);
         const float den = ci + eta_rel * co;
-        if (fabsf(den) < 1.0e-6f) return false;
+        if (fabsf(den) < 1.0e-6f) return kNoSample;
       }
-      return finalize(s, wi, kFlagGlossy | kFlagTransmission, importance, want_rev, out);
+      return rough_direction(wi, kFlagGlossy | kFlagTransmission, out);
     }
   }
   const float eta_rel = m.teta_rel[s.face];
   if (!rough) {
     V3 wi;
-    if (!refract_z(wo, eta_rel, wi)) return false;
+    if (!refract_z(wo, eta_rel, wi)) return kNoSample;
     const float fr = spec_fresnel(m, s.face, fabsf(wo.z));
     const float scale = importance ? 1.0f : 1.0f / (eta_rel * eta_rel);
     out.weight = (weights_below(s, one).btdf * one * (1.0f - fr) * scale) / p_lobe;
     out.wi = wi;
     out.pdf = p_lobe;
     out.flags = kFlagDelta | kFlagTransmission;
-    return true;
+    return kSampled;
   }
   const DevMsFace& fm = m.ms[0][s.face];
   const float ss_p = fm.trans_ss / fm.trans_total;
@@ -1191,26 +1201,27 @@ static __device__ __noinline__ bool sample_btdf(const OpbrVertex& s, float p_lob
   } else {
     const float uu = ss_p > 0.0f ? u0 / ss_p : 0.0f;
     V3 wm;
-    if (!sample_wm_vndf(wo, m.spec_ax, m.spec_ay, uu, u1, wm)) return false;
+    if (!sample_wm_vndf(wo, m.spec_ax, m.spec_ay, uu, u1, wm)) return kNoSample;
     const float co = dot(wo, wm);
-    if (co <= 0.0f) return false;
-    if (!refract_about(wo, wm, eta_rel, wi)) return false;
-    if (wi.z >= 0.0f) return false;
+    if (co <= 0.0f) return kNoSample;
+    if (!refract_about(wo, wm, eta_rel, wi)) return kNoSample;
+    if (wi.z >= 0.0f) return kNoSample;
     const float ci = dot(wi, wm);
     const float den = ci + eta_rel * co;
-    if (fabsf(den) < 1.0e-6f) return false;
+    if (fabsf(den) < 1.0e-6f) return kNoSample;
   }
-  return finalize(s, wi, kFlagGlossy | kFlagTransmission, importance, want_rev, out);
+  return rough_direction(wi, kFlagGlossy | kFlagTransmission, out);
 }
 
-// OpenPbrBsdf::sample (open_pbr.rs:298-332) in the shading frame.
-static __device__ __noinline__ bool sample(const OpbrVertex& s, float u_lobe, float u0, float u1, Sample& out,
-                                           bool importance = false, bool want_rev = false,
-                                           const float* ux = nullptr) {
+// The first half of OpenPbrBsdf::sample (open_pbr.rs:298-332) in the shading
+// frame: picks a lobe and a direction.
+static __device__ __noinline__ SampleStep sample_dir(const OpbrVertex& s, float u_lobe, float u0, float u1,
+                                                     Sample& out, bool importance = false,
+                                                     const float* ux = nullptr) {
   const DevOpenPbr& m = *s.m;
   const V3 wo = s.wo;
   out.lock = -1.0f;
-  if (!(wo.z > 0.0f) || s.q_total <= 0.0f) return false;
+  if (!(wo.z > 0.0f) || s.q_total <= 0.0f) return kNoSample;
   // pick_lobe over (coat, metal, spec_brdf, spec_btdf, fuzz, diff_brdf, diff_btdf = 0)
   float u = u_lobe * s.q_total;
   int lobe;
@@ -1234,21 +1245,20 @@ static __device__ __noinline__ bool sample(const OpbrVertex& s, float u_lobe, fl
     lobe = 4;
     pl = s.q_diff;
   } else {
-    return false;  // diffuse transmission: probability zero
+    return kNoSample;  // diffuse transmission: probability zero
   }
   const float p_lobe = pl / s.q_total;
-  if (p_lobe <= 0.0f) return false;
+  if (p_lobe <= 0.0f) return kNoSample;
   if (lobe == 5) {
     const float zeros[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    return sample_btdf(s, p_lobe, u0, u1, out, importance, want_rev, ux ? ux : zeros);
+    return sample_btdf(s, p_lobe, u0, u1, out, importance, ux ? ux : zeros);
   }
   if (lobe == 3 || lobe == 4) {
     V3 wi;
     const bool ok = lobe == 3 ? fuzz_sample_dir(m.fuzz_roughness, wo, u0, u1, wi)
                               : eon_sample_dir(m.eon_r, m.eon_r_pow01, wo, u0, u1, wi);
-    if (!ok) return false;
-    return finalize(s, wi, lobe == 3 ? (kFlagGlossy | kFlagReflection) : (kFlagDiffuse | kFlagReflection),
-                    importance, want_rev, out);
+    if (!ok) return kNoSample;
+    return rough_direction(wi, lobe == 3 ? (kFlagGlossy | kFlagReflection) : (kFlagDiffuse | kFlagReflection), out);
   }
   const bool rough = lobe == 0 ? (m.flags & kOpbrCoatRough) != 0
                                : (lobe == 1 ? (m.flags & kOpbrMetalRough) != 0 : (m.flags & kOpbrSpecRough) != 0);
@@ -1269,15 +1279,15 @@ static __device__ __noinline__ bool sample(const OpbrVertex& s, float u_lobe, fl
     out.wi = wi;
     out.pdf = p_lobe;
     out.flags = kFlagDelta | kFlagReflection;
-    return true;
+    return kSampled;
   }
   // rough thin-walled specular: GGX single scattering only (open_pbr.rs:1615-1628)
   if (lobe == 2 && (m.flags & kOpbrThinWalled)) {
     V3 wm;
-    if (!sample_wm_bounded_vndf(wo, m.spec_ax, m.spec_ay, u0, u1, wm)) return false;
+    if (!sample_wm_bounded_vndf(wo, m.spec_ax, m.spec_ay, u0, u1, wm)) return kNoSample;
     const V3 wi = reflect_local(wo, wm);
-    if (wi.z <= 0.0f) return false;
-    return finalize(s, wi, kFlagGlossy | kFlagReflection, importance, want_rev, out);
+    if (wi.z <= 0.0f) return kNoSample;
+    return rough_direction(wi, kFlagGlossy | kFlagReflection, out);
   }
   // rough: GGX single scattering or cosine multiple scattering
   float ss, tot, ax, ay;
@@ -1301,11 +1311,20 @@ static __device__ __noinline__ bool sample(const OpbrVertex& s, float u_lobe, fl
   } else {
     const float uu = ss_p > 0.0f ? u0 / ss_p : 0.0f;
     V3 wm;
-    if (!sample_wm_bounded_vndf(wo, ax, ay, uu, u1, wm)) return false;
+    if (!sample_wm_bounded_vndf(wo, ax, ay, uu, u1, wm)) return kNoSample;
     wi = reflect_local(wo, wm);
-    if (wi.z <= 0.0f) return false;
+    if (wi.z <= 0.0f) return kNoSample;
   }
-  return finalize(s, wi, kFlagGlossy | kFlagReflection, importance, want_rev, out);
+  return rough_direction(wi, kFlagGlossy | kFlagReflection, out);
+}
+
+// OpenPbrBsdf::sample: the direction, then a rough sample's value and pdf.
+static __device__ __noinline__ bool sample(const OpbrVertex& s, float u_lobe, float u0, float u1, Sample& out,
+                                           bool importance = false, bool want_rev = false,
+                                           const float* ux = nullptr) {
+  const SampleStep r = sample_dir(s, u_lobe, u0, u1, out, importance, ux);
+  if (r != kRough) return r == kSampled;
+  return finalize(s, out.wi, out.flags, importance, want_rev, out);
 }
 
 }  // namespace opbr

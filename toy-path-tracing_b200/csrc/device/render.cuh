@@ -189,25 +189,16 @@ __device__ __forceinline__ bool opbr_sample_side_ok(const Vertex& v, V3 wi, uint
 }
 
 // OpenPbrMaterial::sample (material/open_pbr.rs:489-563) in radiance transport
-// (modified_bsdf_sample_weight leaves the weight unchanged there).
-static __device__ __noinline__ bool openpbr_sample(const DevRenderData& d, uint32_t opbr_index, const Vertex& v,
-                                            float u_lobe, float u0, float u1, const float* ux, BsdfSampleOut& s) {
+// (modified_bsdf_sample_weight leaves the weight unchanged there), up to the
+// BSDF's state at the vertex; false: no sample.
+static __device__ __noinline__ bool openpbr_begin(const DevRenderData& d, uint32_t opbr_index, const Vertex& v,
+                                                  opbr::OpbrVertex& ov) {
   if (dot(v.wo, v.ng) <= 0.0f) return false;
   const V3 wo_l = normalize_or_zero(to_local(v.frame, v.wo));
   if (wo_l.z <= 0.0f) return false;
-  opbr::OpbrVertex ov;
   opbr::init_vertex(ov, d.openpbr + opbr_index, d.cec_e, d.dec_e, wo_l, v.front, fabsf(wo_l.z));
   ov.thr = v.thr;
   ov.lock = v.lock;
-  opbr::Sample bs;
-  if (!opbr::sample(ov, u_lobe, u0, u1, bs, false, false, ux)) return false;
-  const V3 wi = to_world(v.frame, bs.wi);
-  if (!opbr_sample_side_ok(v, wi, bs.flags)) return false;
-  s.wi = wi;
-  s.weight = bs.weight;
-  s.pdf = bs.pdf;
-  s.delta = (bs.flags & opbr::kFlagDelta) != 0;
-  s.lock = bs.lock;
   return true;
 }
 
@@ -239,19 +230,44 @@ __device__ __forceinline__ void extra_randoms(const DevRenderData& d, const DevM
 }
 
 // Material::sample for the BSDF materials in scope, with the vertex's
-// MaterialSampleRandoms (lobe at offset 5, direction at offset 7).
+// MaterialSampleRandoms (lobe at offset 5, direction at offset 7).  Every thread
+// that calls it gets past every `sync` call, `act` or not: a kernel whose warps
+// share their instruction fetches by running in step passes its barrier.
+struct NoSync {
+  __device__ __forceinline__ void operator()() const {}
+};
+template <class Sync>
 __device__ __forceinline__ bool material_sample(const DevRender& S, const DevMaterialRec& m, const Vertex& v,
-                                                const PathSamplerDev& ps, uint32_t depth, BsdfSampleOut& s) {
-  float ud0, ud1;
-  if (m.kind == kDevOpenPbr) {
-    float u_lobe;
+                                                const PathSamplerDev& ps, uint32_t depth, BsdfSampleOut& s, bool act,
+                                                Sync sync) {
+  const bool open_pbr = act && m.kind == kDevOpenPbr;
+  float ud0, ud1, u_lobe, ux[4];
+  if (open_pbr) {
     ps.sample_2d_1d(vertex_dim(depth, kOffDir), vertex_dim(depth, kOffLobe), ud0, ud1, u_lobe);
-    float ux[4];
     extra_randoms(S.d, m, v, ps, depth, ux);
-    return openpbr_sample(S.d, m.openpbr, v, u_lobe, ud0, ud1, ux, s);
+  } else if (act) {
+    ps.sample_2d(vertex_dim(depth, kOffDir), ud0, ud1);
   }
-  ps.sample_2d(vertex_dim(depth, kOffDir), ud0, ud1);
-  return lambert_sample(m, v, ud0, ud1, s);
+  sync();
+  opbr::OpbrVertex ov;
+  opbr::Sample bs;
+  opbr::SampleStep step = opbr::kNoSample;
+  const bool begun = open_pbr && openpbr_begin(S.d, m.openpbr, v, ov);
+  sync();
+  if (begun) step = opbr::sample_dir(ov, u_lobe, ud0, ud1, bs, false, ux);
+  sync();
+  if (step == opbr::kRough) step = opbr::finalize(ov, bs.wi, bs.flags, false, false, bs) ? opbr::kSampled : opbr::kNoSample;
+  sync();
+  if (!open_pbr) return act && lambert_sample(m, v, ud0, ud1, s);
+  if (step == opbr::kNoSample) return false;
+  const V3 wi = to_world(v.frame, bs.wi);
+  if (!opbr_sample_side_ok(v, wi, bs.flags)) return false;
+  s.wi = wi;
+  s.weight = bs.weight;
+  s.pdf = bs.pdf;
+  s.delta = (bs.flags & opbr::kFlagDelta) != 0;
+  s.lock = bs.lock;
+  return true;
 }
 
 // ---------------------------------------------------------------------------

@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(kRenderBlock, TPT_MK_MINB) render_mis_kernel(c
         }
         bool alive = false;
         BsdfSampleOut s;
-        if (material_sample(S, m, v, ps, depth, s)) {
+        if (material_sample(S, m, v, ps, depth, s, true, NoSync())) {
           beta = beta * s.weight;
           if (s.lock >= 0.0f) lock = s.lock;
           alive = true;

@@ -11,10 +11,11 @@ cudaError_t launch_wf_shade(const DevGeometry& geo, const DevRenderData& rd, con
   if (A) return launch_wf_shade_adjoint(geo, rd, P, B, cur, s, *A);
   DevRender S{geo, rd};
   const DevAdjoint none{};
+  const int bs = shade_launch_block(block);
   if (rd.num_extra_lights > 0)
-    wf_shade<false, false, true><<<grid_for(B.capacity, block), block, 0, s>>>(S, P, B, cur, none, nullptr);
+    wf_shade<false, false, true><<<grid_for(B.capacity, bs), bs, 0, s>>>(S, P, B, cur, none, nullptr);
   else
-    wf_shade<false, false, false><<<grid_for(B.capacity, block), block, 0, s>>>(S, P, B, cur, none, nullptr);
+    wf_shade<false, false, false><<<grid_for(B.capacity, bs), bs, 0, s>>>(S, P, B, cur, none, nullptr);
   return cudaGetLastError();
 }
 

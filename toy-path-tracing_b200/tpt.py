@@ -447,7 +447,7 @@ class Context:
         return out.cpu().numpy(), seeds.cpu().numpy().view(np.uint32)
 
     def set_shade_block(self, threads: int):
-        """`tpt_context_set_shade_block`: 128 or 256 threads per shade block."""
+        """`tpt_context_set_shade_block`: 128 threads per shade block, or 256 for full blocks."""
         _check(lib().tpt_context_set_shade_block(self.h, int(threads)), self)
 
     def render_batch_device(self, jobs, out_ptrs, stream=None):
