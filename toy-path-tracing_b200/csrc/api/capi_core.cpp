@@ -485,7 +485,9 @@ tpt_status tpt_scene_upload(tpt_context* ctx, const tpt_scene_desc* desc, tpt_sc
     mesh_tri_base[m] = (uint32_t)n_tris;
     mesh_root[m] = qnn ? 0u : (kLeafFlag | ((uint32_t)qpn << 24));
     tri_counts[m] = (uint32_t)ntri;
-    for (uint64_t i = 0; i < qnn; ++i) nodes.push_back(to_dev(qn[i]));
+    nodes.resize(mesh_node_base[m] + qnn);
+    for (uint64_t i = 0; i < qnn; ++i) nodes[mesh_node_base[m] + i] = to_dev(qn[i]);
+    tris.resize((n_tris + qpn + 1) / 2);
     for (uint64_t k = 0; k < qpn; ++k) {
       uint32_t t = qp[k];
       Vec3f a = pos(md.indices[3 * (size_t)t]), b = pos(md.indices[3 * (size_t)t + 1]),
@@ -498,9 +500,8 @@ tpt_status tpt_scene_upload(tpt_context* ctx, const tpt_scene_desc* desc, tpt_sc
       uint32_t tb = t;
       float tf;
       std::memcpy(&tf, &tb, 4);
+      DevTriPair& d = tris[n_tris >> 1];
       const uint32_t half = (uint32_t)(n_tris++ & 1u);
-      if (half == 0) tris.push_back(DevTriPair{});
-      DevTriPair& d = tris.back();
       d.v01[half][0] = make_float4(a.x, a.y, a.z, tf);
       d.v01[half][1] = make_float4(b.x, b.y, b.z, l2 == 0.0f ? 1.0f : 0.0f);
       d.v2[half] = make_float4(c.x, c.y, c.z, 0.0f);

@@ -58,35 +58,34 @@ struct MatSample {
   float lock;  // wavelength lock set by the sample (< 0: none)
 };
 
-// Material::sample with pdf_rev
-static __device__ __noinline__ bool material_sample_rev(const DevRender& S, const DevMaterialRec& m, const Vertex& v,
-                                                       float u_lobe, float u0, float u1, const float* ux,
-                                                       bool importance, MatSample& s) {
-  s.lock = -1.0f;
-  if (m.kind == kDevLambert) {
-    const V3 wo_l = normalize_or_zero(to_local(v.frame, v.wo));
-    if (wo_l.z <= 0.0f) return false;
-    const V3 wi_l = opbr::sample_cosine_hemisphere(u0, u1);
-    const float pdf = lambert_bsdf_pdf(wo_l, wi_l);
-    if (pdf <= 0.0f) return false;
-    const V3 wi = to_world(v.frame, wi_l);
-    s.weight = modified_weight(v, wi, V3{m.rho[0], m.rho[1], m.rho[2]}, false, importance);
-    s.wi = wi;
-    s.pdf = pdf;
-    s.pdf_rev = lambert_bsdf_pdf(wi_l, wo_l);
-    s.delta = false;
-    return dot(wi, v.ng) > kGeomCosEps;
+// Material::sample with pdf_rev and the vertex's MaterialSampleRandoms.  Every
+// thread that calls it gets past every `sync` call, `act` or not (material_sample).
+template <class Sync>
+__device__ __forceinline__ bool material_sample_rev(const DevRender& S, const DevMaterialRec& m, const Vertex& v,
+                                                    const PathSamplerDev& ps, uint32_t depth, bool importance,
+                                                    MatSample& s, bool act, Sync sync) {
+  const bool open_pbr = act && m.kind == kDevOpenPbr;
+  float ud0, ud1, u_lobe, ux[4];
+  if (open_pbr) {
+    ps.sample_2d_1d(vertex_dim(depth, kOffDir), vertex_dim(depth, kOffLobe), ud0, ud1, u_lobe);
+    extra_randoms(S.d, m, v, ps, depth, ux);
+  } else if (act) {
+    ps.sample_2d(vertex_dim(depth, kOffDir), ud0, ud1);
   }
-  if (m.kind == kDevOpenPbr) {
-    if (dot(v.wo, v.ng) <= 0.0f) return false;
-    const V3 wo_l = normalize_or_zero(to_local(v.frame, v.wo));
-    if (wo_l.z <= 0.0f) return false;
-    opbr::OpbrVertex ov;
-    opbr::init_vertex(ov, S.d.openpbr + m.openpbr, S.d.cec_e, S.d.dec_e, wo_l, v.front, fabsf(wo_l.z));
-    ov.thr = v.thr;
-    ov.lock = v.lock;
-    opbr::Sample bs;
-    if (!opbr::sample(ov, u_lobe, u0, u1, bs, importance, true, ux)) return false;
+  s.lock = -1.0f;
+  sync();
+  opbr::OpbrVertex ov;
+  opbr::Sample bs;
+  opbr::SampleStep step = opbr::kNoSample;
+  const bool begun = open_pbr && openpbr_begin(S.d, m.openpbr, v, ov);
+  sync();
+  if (begun) step = opbr::sample_dir(ov, u_lobe, ud0, ud1, bs, importance, ux);
+  sync();
+  if (step == opbr::kRough)
+    step = opbr::finalize(ov, bs.wi, bs.flags, importance, true, bs) ? opbr::kSampled : opbr::kNoSample;
+  sync();
+  if (open_pbr) {
+    if (step == opbr::kNoSample) return false;
     s.lock = bs.lock;
     const V3 wi = to_world(v.frame, bs.wi);
     if (!opbr_sample_side_ok(v, wi, bs.flags)) return false;
@@ -97,7 +96,19 @@ static __device__ __noinline__ bool material_sample_rev(const DevRender& S, cons
     s.pdf_rev = bs.pdf_rev;
     return true;
   }
-  return false;  // pure emitter
+  if (!act || m.kind != kDevLambert) return false;  // a pure emitter has no sample
+  const V3 wo_l = normalize_or_zero(to_local(v.frame, v.wo));
+  if (wo_l.z <= 0.0f) return false;
+  const V3 wi_l = opbr::sample_cosine_hemisphere(ud0, ud1);
+  const float pdf = lambert_bsdf_pdf(wo_l, wi_l);
+  if (pdf <= 0.0f) return false;
+  const V3 wi = to_world(v.frame, wi_l);
+  s.weight = modified_weight(v, wi, V3{m.rho[0], m.rho[1], m.rho[2]}, false, importance);
+  s.wi = wi;
+  s.pdf = pdf;
+  s.pdf_rev = lambert_bsdf_pdf(wi_l, wo_l);
+  s.delta = false;
+  return dot(wi, v.ng) > kGeomCosEps;
 }
 
 // ---- path vertices ---------------------------------------------------------
@@ -218,34 +229,51 @@ struct BdConnection {
   V3 c, origin, dir;
   float dist;
 };
+// `act` and `sync` as in material_sample: the vertices are read only with `act`.
+template <class Sync>
 __device__ __forceinline__ int bdpt_connect_prepare(const DevRender& S, const BdVertex& lv, const BdVertex& cv,
-                                                    BdConnection& out) {
-  const V3 delta = cv.v.p - lv.v.p;
-  const float dist2 = length_sq(delta);
-  if (dist2 <= 0.0f) return 0;
-  const float dist = sqrtf(dist2);
-  const V3 w_lc = delta / dist;
-  const V3 w_cl = -w_lc;
-  out.origin = offset_origin(lv.v.p, lv.v.ng, w_lc);
-  out.dir = w_lc;
-  out.dist = dist;
-  out.c = V3{0.0f, 0.0f, 0.0f};
-  const DevMaterialRec cm = S.d.mats[__ldg(&S.d.inst[cv.v.inst].material)];
-  const V3 f_cam = material_eval(S, cm, cv.v, w_cl, false);
-  if (length_sq(f_cam) == 0.0f) return 1;
-  V3 f_light;
-  if (lv.flags & kBdLight) {
-    if (dot(lv.v.ng, w_lc) <= 0.0f) return 1;
-    f_light = V3{1.0f, 1.0f, 1.0f};
-  } else {
-    const DevMaterialRec lm = S.d.mats[__ldg(&S.d.inst[lv.v.inst].material)];
-    f_light = material_eval(S, lm, lv.v, w_lc, true);
+                                                    BdConnection& out, bool act, Sync sync) {
+  int r = 0;
+  float dist2 = 0.0f;
+  V3 w_lc, w_cl, f_cam, f_light;
+  if (act) {
+    const V3 delta = cv.v.p - lv.v.p;
+    dist2 = length_sq(delta);
+    if (!(dist2 <= 0.0f)) {
+      const float dist = sqrtf(dist2);
+      w_lc = delta / dist;
+      w_cl = -w_lc;
+      out.origin = offset_origin(lv.v.p, lv.v.ng, w_lc);
+      out.dir = w_lc;
+      out.dist = dist;
+      out.c = V3{0.0f, 0.0f, 0.0f};
+      r = 2;
+    }
   }
-  if (length_sq(f_light) == 0.0f) return 1;
-  const float g = fabsf(dot(lv.v.ng, w_lc)) * fabsf(dot(cv.v.ng, w_cl)) / dist2;
-  if (g <= 0.0f) return 1;
-  out.c = lv.v.thr * f_light * g * f_cam * cv.v.thr;
-  return 2;
+  sync();
+  if (r == 2) {
+    const DevMaterialRec cm = S.d.mats[__ldg(&S.d.inst[cv.v.inst].material)];
+    f_cam = material_eval(S, cm, cv.v, w_cl, false);
+    if (length_sq(f_cam) == 0.0f) r = 1;
+  }
+  sync();
+  if (r == 2) {
+    if (lv.flags & kBdLight) {
+      f_light = V3{1.0f, 1.0f, 1.0f};
+      if (dot(lv.v.ng, w_lc) <= 0.0f) r = 1;
+    } else {
+      const DevMaterialRec lm = S.d.mats[__ldg(&S.d.inst[lv.v.inst].material)];
+      f_light = material_eval(S, lm, lv.v, w_lc, true);
+      if (length_sq(f_light) == 0.0f) r = 1;
+    }
+  }
+  sync();
+  if (r == 2) {
+    const float g = fabsf(dot(lv.v.ng, w_lc)) * fabsf(dot(cv.v.ng, w_cl)) / dist2;
+    if (g <= 0.0f) return 1;
+    out.c = lv.v.thr * f_light * g * f_cam * cv.v.thr;
+  }
+  return r;
 }
 
 // The subpaths and connections below are warp-synchronous: every lane of the
@@ -281,21 +309,23 @@ __device__ __forceinline__ void camera_state_init(BdCamState& c, bool valid) {
 // whether the vertex took such a light sample (bdpt.rs:207-221): its
 // contribution, times the path throughput, counts into L once the shadow ray
 // of `dp` is found unoccluded, before the next iteration adds anything.
+// The iteration is split at the BSDF sample (material_sample_rev): camera_vertex
+// returns whether one is to be drawn at (v, m), camera_continue takes it.
 template <class Stack>
-__device__ __forceinline__ void camera_step(const DevRender& S, const RenderLaunch& P, const PathSamplerDev& ps,
-                                            uint32_t depth, const TraceResult& h, V3& ro, V3& rd, BdVertex* vs,
-                                            BdCamState& c, V3& L, bool& nee, DirectPrep& dp) {
+__device__ __forceinline__ bool camera_vertex(const DevRender& S, const PathSamplerDev& ps, uint32_t depth,
+                                              const TraceResult& h, V3 rd, BdVertex* vs, BdCamState& c, V3& L,
+                                              bool& nee, DirectPrep& dp, Vertex& v, DevMaterialRec& m) {
   nee = false;
   if (h.tri < 0) {
     // emitted_radiance_from_infinite_hit (bdpt.rs:466-486)
     if (S.d.has_env) L = L + c.beta * env_escape(S.d, rd, c.count_emission, false, c.pending_pdf);
     c.alive = false;
-    return;
+    return false;
   }
-  Vertex v = shade_hit<Stack>(S, h, rd);
+  v = shade_hit<Stack>(S, h, rd);
   v.thr = c.beta;  // the path state the vertex keeps (bdpt.rs:177-178)
   v.lock = c.lock;
-  const DevMaterialRec m = S.d.mats[__ldg(&S.d.inst[v.inst].material)];
+  m = S.d.mats[__ldg(&S.d.inst[v.inst].material)];
   BdVertex& pv = vs[c.n];
   pv.v = v;
   pv.pdf_fwd = c.have_pending ? solid_angle_to_area(c.pending_pdf, c.pending_from, v.p, v.ng) : 0.0f;
@@ -309,21 +339,23 @@ __device__ __forceinline__ void camera_step(const DevRender& S, const RenderLaun
   }
   if (m.kind == kDevEmissive) {
     c.alive = false;  // pure emitter: sample() is None
-    return;
+    return false;
   }
   if (S.d.num_extra_lights > 0) {  // direct_non_area_light_contribution
     nee = prepare_direct<true, kDirectBdptNonArea>(S, m, v, ps, depth, dp);
     if (nee) dp.contrib = c.beta * dp.contrib;
   }
-  float ud0, ud1, u_lobe = 0.0f, ux[4];
-  if (m.kind == kDevOpenPbr) ps.sample_2d_1d(vertex_dim(depth, kOffDir), vertex_dim(depth, kOffLobe), ud0, ud1, u_lobe);
-  else ps.sample_2d(vertex_dim(depth, kOffDir), ud0, ud1);
-  extra_randoms(S.d, m, v, ps, depth, ux);
-  MatSample s;
-  if (!material_sample_rev(S, m, v, u_lobe, ud0, ud1, ux, false, s)) {
+  return true;
+}
+__device__ __forceinline__ void camera_continue(const PathSamplerDev& ps, uint32_t depth, const Vertex& v,
+                                                bool sampled, const MatSample& s, V3& ro, V3& rd, BdVertex* vs,
+                                                BdCamState& c) {
+  if (!sampled) {
     c.alive = false;
     return;
   }
+  const uint32_t n = c.n;
+  BdVertex& pv = vs[n - 1];
   if (s.lock >= 0.0f) c.lock = s.lock;
   pv.flags = s.delta ? kBdDelta : kBdConnectible;
   if (n >= 2) vs[n - 2].pdf_rev = solid_angle_to_area(s.pdf_rev, v.p, vs[n - 2].v.p, vs[n - 2].v.ng);
@@ -362,7 +394,15 @@ __device__ __forceinline__ uint32_t bdpt_camera_subpath(const DevRender& S, Stac
       trace_ray_ww<0>(S.geo, st, live, ro.x, ro.y, ro.z, rd.x, rd.y, rd.z, __int_as_float(0x7f800000), h, err, aux);
     bool nee = false;
     DirectPrep dp;
-    if (c.alive) camera_step<Stack>(S, P, ps, depth, h, ro, rd, vs, c, L, nee, dp);
+    if (c.alive) {
+      Vertex v;
+      DevMaterialRec m;
+      MatSample s;
+      if (camera_vertex<Stack>(S, ps, depth, h, rd, vs, c, L, nee, dp, v, m)) {
+        const bool sampled = material_sample_rev(S, m, v, ps, depth, false, s, true, NoSync());
+        camera_continue(ps, depth, v, sampled, s, ro, rd, vs, c);
+      }
+    }
     const unsigned sm = __ballot_sync(0xffffffffu, nee);
     if (sm) {  // the light samples' shadow rays (unoccluded, integrator/mod.rs:239-265)
       TraceResult hs;
@@ -443,37 +483,39 @@ struct BdLightState {
 
 static_assert(sizeof(BdCamState) <= kBdStateBytes && sizeof(BdLightState) <= kBdStateBytes, "BDPT loop states");
 
-// One iteration of the light loop (bdpt.rs:264-385) after its ray was traced to h.
+// One iteration of the light loop (bdpt.rs:264-385) after its ray was traced to h,
+// split as the camera loop's.
 template <class Stack>
-__device__ __forceinline__ void light_step(const DevRender& S, const PathSamplerDev& ps, uint32_t depth,
-                                           const TraceResult& h, V3& ro, V3& rd, BdVertex* vs, BdLightState& l) {
+__device__ __forceinline__ bool light_vertex(const DevRender& S, const TraceResult& h, V3 rd, BdVertex* vs,
+                                             BdLightState& l, Vertex& v, DevMaterialRec& m) {
   if (h.tri < 0) {
     l.alive = false;
-    return;
+    return false;
   }
-  Vertex v = shade_hit<Stack>(S, h, rd);
+  v = shade_hit<Stack>(S, h, rd);
   v.thr = l.beta;  // bdpt.rs:344-345
   v.lock = l.lock;
-  const DevMaterialRec m = S.d.mats[__ldg(&S.d.inst[v.inst].material)];
+  m = S.d.mats[__ldg(&S.d.inst[v.inst].material)];
   BdVertex& pv = vs[l.n];
   pv.v = v;
   pv.pdf_fwd = solid_angle_to_area(l.pending_pdf, l.pending_from, v.p, v.ng);
   pv.pdf_rev = 0.0f;
   pv.flags = m.kind != kDevEmissive ? kBdConnectible : 0u;
-  const uint32_t n = ++l.n;
+  ++l.n;
   if (m.kind == kDevEmissive) {
     l.alive = false;
-    return;
+    return false;
   }
-  float ud0, ud1, u_lobe = 0.0f, ux[4];
-  if (m.kind == kDevOpenPbr) ps.sample_2d_1d(vertex_dim(depth, kOffDir), vertex_dim(depth, kOffLobe), ud0, ud1, u_lobe);
-  else ps.sample_2d(vertex_dim(depth, kOffDir), ud0, ud1);
-  extra_randoms(S.d, m, v, ps, depth, ux);
-  MatSample s;
-  if (!material_sample_rev(S, m, v, u_lobe, ud0, ud1, ux, true, s)) {
+  return true;
+}
+__device__ __forceinline__ void light_continue(const Vertex& v, bool sampled, const MatSample& s, V3& ro, V3& rd,
+                                               BdVertex* vs, BdLightState& l) {
+  if (!sampled) {
     l.alive = false;
     return;
   }
+  const uint32_t n = l.n;
+  BdVertex& pv = vs[n - 1];
   if (s.lock >= 0.0f) l.lock = s.lock;
   pv.flags = s.delta ? kBdDelta : kBdConnectible;
   vs[n - 2].pdf_rev = solid_angle_to_area(s.pdf_rev, v.p, vs[n - 2].v.p, vs[n - 2].v.ng);
@@ -501,7 +543,15 @@ __device__ __forceinline__ uint32_t bdpt_light_subpath(const DevRender& S, Stack
     if (aux && l.alive) *aux = aux_from_seed(ps, (int)depth);
     if (l.alive)
       trace_ray_ww<0>(S.geo, st, live, ro.x, ro.y, ro.z, rd.x, rd.y, rd.z, __int_as_float(0x7f800000), h, err, aux);
-    if (l.alive) light_step<Stack>(S, ps, depth, h, ro, rd, vs, l);
+    if (l.alive) {
+      Vertex v;
+      DevMaterialRec m;
+      MatSample s;
+      if (light_vertex<Stack>(S, h, rd, vs, l, v, m)) {
+        const bool sampled = material_sample_rev(S, m, v, ps, depth, true, s, true, NoSync());
+        light_continue(v, sampled, s, ro, rd, vs, l);
+      }
+    }
   }
   return l.n;
 }
@@ -531,7 +581,7 @@ __device__ V3 trace_bdpt(const DevRender& S, Stack& st, bool valid, const Render
       li = k / nc;
       ci = k - li * nc;
       if ((lig[li].flags & kBdConnectible) && (cam[ci].flags & kBdConnectible)) {
-        prep = bdpt_connect_prepare(S, lig[li], cam[ci], cn);
+        prep = bdpt_connect_prepare(S, lig[li], cam[ci], cn, true, NoSync());
         want = prep == 2 || (alpha && prep == 1);
       }
     }

@@ -35,12 +35,17 @@
 namespace tpt {
 
 constexpr int kBdWfBlock = 128;
-#ifndef TPT_BD_STEP_MINB
-// bd_step's minimum resident blocks per SM: 4 caps it at 128 registers (from
-// 168, a few hundred bytes of spills), 16 warps per SM instead of 12: 6 % less
-// BDPT time on the large scene
-#define TPT_BD_STEP_MINB 4
-#endif
+// bd_step and bd_connect evaluate whole BSDFs per thread, thousands of
+// instructions nearly without loops, and are bound by instruction fetches as the
+// path tracer's shade stage is: their blocks are large and pass a barrier between
+// the parts, so that a block's warps share each fetch.  Measured (2.1M triangles,
+// path length 10, 480x270 at 8 / 1 spp, ms): 4 blocks of 128 per SM, no barriers
+// 21.5 / 5.59; 2 x 384 no barriers 20.0 / 5.63, with them 18.9 / 5.63; 1 x 640
+// 19.0 / 5.62; 2 x 512 18.4 / 5.58.
+constexpr int kBdShadeBlock = 512, kBdShadeMinBlocks = 2;
+struct BlockSync {
+  __device__ __forceinline__ void operator()() const { __syncthreads(); }
+};
 
 // Warp-exclusive prefix sum of `v` (all lanes call); returns the lane's offset
 // and the warp total in `total`.
@@ -133,46 +138,71 @@ __global__ void __launch_bounds__(kBdWfBlock) bd_init(const __grid_constant__ De
 
 // Step `step` of both loops: camera rays of depth `step`, light rays of depth
 // step + 1, traced into the hit arrays; the next rays into queue cur ^ 1.
-__global__ void __launch_bounds__(kBdWfBlock, TPT_BD_STEP_MINB) bd_step(const __grid_constant__ DevRender S,
-                                                  const __grid_constant__ RenderLaunch P, BdWfBuffers B,
-                                                      uint64_t first_path, uint32_t step, int cur) {
+__global__ void __launch_bounds__(kBdShadeBlock, kBdShadeMinBlocks)
+    bd_step(const __grid_constant__ DevRender S, const __grid_constant__ RenderLaunch P, BdWfBuffers B,
+            uint64_t first_path, uint32_t step, int cur) {
+  const BlockSync sync;
   const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t S_cap = B.sample_capacity, Q = 2 * S_cap;
-  if (j < S_cap ? j >= B.counts[2 + cur] : j - S_cap >= B.counts[4 + cur]) return;
-  const uint32_t tag = B.q_tag[cur][j];
-  const uint32_t i = tag & ~kLightTag;
-  const bool light = (tag & kLightTag) != 0;
-  uint32_t px, py;
-  const PathSamplerDev ps = sampler_of(P, first_path + i, px, py);
-  TraceResult h;
-  h.tri = B.h_tri[j];
-  h.inst = B.h_inst[j];
-  h.t = B.h_t[j];
-  h.b0 = B.h_bary[j];
-  h.b1 = B.h_bary[Q + j];
-  h.b2 = B.h_bary[2 * Q + j];
-  const float* r = B.q_ray[cur];
-  V3 ro = V3{r[j], r[Q + j], r[2 * Q + j]};
-  V3 rd = V3{r[3 * Q + j], r[4 * Q + j], r[5 * Q + j]};
-  BdVertex* cam = B.verts + (size_t)i * 2 * B.max_vertices;
-  bool next = false;
-  bool nee = false;
+  const bool light = j >= S_cap;
+  const bool valid = light ? j < Q && j - S_cap < B.counts[4 + cur] : j < B.counts[2 + cur];
+  if (!__syncthreads_or(valid)) return;
+  uint32_t tag = 0, i = 0, depth = 0;
+  PathSamplerDev ps;
+  V3 ro, rd;
+  BdVertex* verts = B.verts;  // of this thread's subpath
+  bool scatters = false, next = false, nee = false;
   DirectPrep dp;
-  if (!light) {
-    BdCamState c = B.cam_state[i];
-    V3 L = V3{B.L0[3 * (size_t)i], B.L0[3 * (size_t)i + 1], B.L0[3 * (size_t)i + 2]};
-    camera_step<int>(S, P, ps, step, h, ro, rd, cam, c, L, nee, dp);
-    B.cam_state[i] = c;
-    B.L0[3 * (size_t)i] = L.x;
-    B.L0[3 * (size_t)i + 1] = L.y;
-    B.L0[3 * (size_t)i + 2] = L.z;
-    next = c.alive && step + 1 < P.max_depth;
-  } else {
-    BdLightState l = B.light_state[i];
-    light_step<int>(S, ps, step + 1, h, ro, rd, cam + B.max_vertices, l);
-    B.light_state[i] = l;
-    next = l.alive && step + 2 < P.max_depth;
+  Vertex v;
+  DevMaterialRec m;
+  if (valid) {
+    tag = B.q_tag[cur][j];
+    i = tag & ~kLightTag;
+    depth = step + (light ? 1u : 0u);
+    verts += (size_t)i * 2 * B.max_vertices + (light ? B.max_vertices : 0u);
+    uint32_t px, py;
+    ps = sampler_of(P, first_path + i, px, py);
+    TraceResult h;
+    h.tri = B.h_tri[j];
+    h.inst = B.h_inst[j];
+    h.t = B.h_t[j];
+    h.b0 = B.h_bary[j];
+    h.b1 = B.h_bary[Q + j];
+    h.b2 = B.h_bary[2 * Q + j];
+    const float* r = B.q_ray[cur];
+    rd = V3{r[3 * Q + j], r[4 * Q + j], r[5 * Q + j]};
+    if (!light) {
+      BdCamState c = B.cam_state[i];
+      V3 L = V3{B.L0[3 * (size_t)i], B.L0[3 * (size_t)i + 1], B.L0[3 * (size_t)i + 2]};
+      scatters = camera_vertex<int>(S, ps, depth, h, rd, verts, c, L, nee, dp, v, m);
+      B.cam_state[i] = c;
+      B.L0[3 * (size_t)i] = L.x;
+      B.L0[3 * (size_t)i + 1] = L.y;
+      B.L0[3 * (size_t)i + 2] = L.z;
+    } else {
+      BdLightState l = B.light_state[i];
+      scatters = light_vertex<int>(S, h, rd, verts, l, v, m);
+      B.light_state[i] = l;
+    }
   }
+  sync();
+  MatSample ms;
+  const bool sampled = material_sample_rev(S, m, v, ps, depth, light, ms, scatters, sync);
+  if (scatters) {  // the subpath state comes back from memory: it need not live through the sampling
+    if (!light) {
+      BdCamState c = B.cam_state[i];
+      camera_continue(ps, depth, v, sampled, ms, ro, rd, verts, c);
+      B.cam_state[i] = c;
+      next = c.alive && step + 1 < P.max_depth;
+    } else {
+      BdLightState l = B.light_state[i];
+      light_continue(v, sampled, ms, ro, rd, verts, l);
+      B.light_state[i] = l;
+      next = l.alive && step + 2 < P.max_depth;
+    }
+  }
+  sync();
+  if (!valid) return;
   const uint32_t q = warp_append1(&B.counts[(light ? 4 : 2) + (cur ^ 1)], next);
   if (next) push_ray(B, cur ^ 1, light ? S_cap + q : q, ro, rd, tag);
   // a camera vertex's light sample: its shadow ray into the visibility queue
@@ -229,9 +259,13 @@ __global__ void __launch_bounds__(kBdWfBlock) bd_pairs(BdWfBuffers B, uint32_t n
   for (uint32_t k = 0; k < np; ++k) B.pair_sample[pbase + k] = i;
 }
 
-__global__ void __launch_bounds__(kBdWfBlock) bd_connect(const __grid_constant__ DevRender S, BdWfBuffers B) {
-  const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= B.counts[0]) return;
+__global__ void __launch_bounds__(kBdShadeBlock, kBdShadeMinBlocks)
+    bd_connect(const __grid_constant__ DevRender S, BdWfBuffers B) {
+  const uint32_t n_pairs = B.counts[0];
+  if (blockIdx.x * blockDim.x >= n_pairs) return;
+  // threads past the end stay for the barriers, on the last pair
+  const bool valid = blockIdx.x * blockDim.x + threadIdx.x < n_pairs;
+  const uint32_t j = valid ? blockIdx.x * blockDim.x + threadIdx.x : n_pairs - 1;
   const uint32_t MD = B.max_vertices;
   const uint32_t i = B.pair_sample[j];
   const uint32_t k = j - B.pair_base[i];
@@ -241,8 +275,9 @@ __global__ void __launch_bounds__(kBdWfBlock) bd_connect(const __grid_constant__
   const BdVertex& lv = cam[MD + li];
   const BdVertex& cv = cam[ci];
   BdConnection cn;
-  bool want = false;
-  if ((lv.flags & kBdConnectible) && (cv.flags & kBdConnectible)) want = bdpt_connect_prepare(S, lv, cv, cn) == 2;
+  const bool act = valid && (lv.flags & kBdConnectible) && (cv.flags & kBdConnectible);
+  const bool want = bdpt_connect_prepare(S, lv, cv, cn, act, BlockSync()) == 2;
+  if (!valid) return;
   B.contrib[3 * (size_t)j] = 0.0f;
   B.contrib[3 * (size_t)j + 1] = 0.0f;
   B.contrib[3 * (size_t)j + 2] = 0.0f;
@@ -304,7 +339,7 @@ __global__ void __launch_bounds__(kBdWfBlock) bd_finalize(BdWfBuffers B, uint32_
   samples[3 * (size_t)i + 2] = L.z;
 }
 
-static inline unsigned grid_of(uint64_t n) { return (unsigned)((n + kBdWfBlock - 1) / kBdWfBlock); }
+static inline unsigned grid_of(uint64_t n, int block = kBdWfBlock) { return (unsigned)((n + block - 1) / block); }
 
 cudaError_t launch_bdpt_wavefront(const DevGeometry& geo, const DevRenderData& rd, const RenderLaunch& P,
                                   const BdWfBuffers& B, uint64_t first_path, uint32_t n, float* samples,
@@ -346,7 +381,7 @@ cudaError_t launch_bdpt_wavefront(const DevGeometry& geo, const DevRenderData& r
       if (e == cudaSuccess) e = ew;
     }
     if (e != cudaSuccess) return e;
-    bd_step<<<grid_of(Q), kBdWfBlock, 0, s>>>(S, P, B, first_path, step, cur);
+    bd_step<<<grid_of(Q, kBdShadeBlock), kBdShadeBlock, 0, s>>>(S, P, B, first_path, step, cur);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if (lights) {  // at most one light sample per sample and step: n <= sample_capacity <= pair_capacity
       e = launch_traverse_strided(geo, B.s_ray, B.pair_capacity, B.pair_capacity, TPT_CLOSEST_HIT, B.s_tri, B.s_t,
@@ -360,7 +395,7 @@ cudaError_t launch_bdpt_wavefront(const DevGeometry& geo, const DevRenderData& r
   }
   bd_pairs<<<grid_of(n), kBdWfBlock, 0, s>>>(B, n);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  bd_connect<<<grid_of(B.pair_capacity), kBdWfBlock, 0, s>>>(S, B);
+  bd_connect<<<grid_of(B.pair_capacity, kBdShadeBlock), kBdShadeBlock, 0, s>>>(S, B);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   e = launch_traverse_strided(geo, B.s_ray, B.pair_capacity, B.pair_capacity, TPT_CLOSEST_HIT, B.s_tri, B.s_t,
                               B.s_inst, nullptr, B.pair_capacity, counter, err, num_sms, s, nullptr, nullptr,
