@@ -6,6 +6,7 @@
 // radiance into the context's sample scratch) and then its adjoint replay over
 // the same paths (wavefront_kernels.cu, ADJ = true), which adds every rough
 // OpenPBR vertex's contribution to per-material FP64 gradients.
+#include <algorithm>
 #include <cstring>
 #include <string>
 
@@ -115,13 +116,20 @@ tpt_status tpt_scene_set_openpbr(tpt_context* ctx, tpt_scene* scene, uint32_t co
     tpt_status st = lower_openpbr_material(ctx, descs[k], &recs[k]);
     if (st) return st;
   }
+  // one copy per run of consecutive table entries (in the list's order, so that
+  // a material listed twice keeps its last entry): each copy costs the host some
+  // 5 us
   DevOpenPbr* table = const_cast<DevOpenPbr*>(scene->render.openpbr);
-  for (uint32_t k = 0; k < count; ++k) {
+  for (uint32_t k = 0; k < count;) {
     const uint32_t t = scene->opbr_of_material[material_ids[k]];
+    uint32_t run = 1;
+    while (k + run < count && scene->opbr_of_material[material_ids[k + run]] == t + run) ++run;
     tpt_status st = cuda_check(
-        ctx, cudaMemcpyAsync(table + t, &recs[k], sizeof(DevOpenPbr), cudaMemcpyHostToDevice, s), "material update");
+        ctx, cudaMemcpyAsync(table + t, &recs[k], run * sizeof(DevOpenPbr), cudaMemcpyHostToDevice, s),
+        "material update");
     if (st) return st;
-    scene->opbr_desc[t] = descs[k];
+    std::copy(descs + k, descs + k + run, scene->opbr_desc.begin() + t);
+    k += run;
   }
   // the records above are pageable host memory: the copies are staged before return
   scene->mat_version++;

@@ -66,6 +66,20 @@ unsigned long long* next_counter(tpt_context* ctx) {
   return ctx->d_counters + k;
 }
 
+tpt_status ensure_device_staging(tpt_context* ctx, size_t bytes) {
+  if (ctx->d_stage_bytes >= bytes) return TPT_OK;
+  if (ctx->d_stage) {
+    cudaStreamSynchronize(ctx->stream);
+    cudaFree(ctx->d_stage);
+  }
+  ctx->d_stage = nullptr;
+  ctx->d_stage_bytes = 0;
+  tpt_status st = cuda_check(ctx, cudaMalloc(&ctx->d_stage, bytes), "cudaMalloc(staging)");
+  if (st) return st;
+  ctx->d_stage_bytes = bytes;
+  return TPT_OK;
+}
+
 }  // namespace tpt
 
 using namespace tpt;
@@ -78,6 +92,64 @@ int host_threads(int requested) {
   return hc ? (int)hc : 1;
 }
 
+// Host copies run together, on several threads when they are large: one core
+// copies about 10 GB/s and takes the page faults of fresh result arrays one by
+// one, a fifth of what the PCIe copies beside it reach.
+struct HostCopies {
+  struct Part {
+    char* dst;
+    const char* src;
+    size_t bytes;
+  };
+  std::vector<Part> parts;
+  size_t total = 0;
+  void add(void* dst, const void* src, size_t bytes) {
+    parts.push_back(Part{(char*)dst, (const char*)src, bytes});
+    total += bytes;
+  }
+  // bytes [from, to) of the parts laid end to end
+  void copy_range(size_t from, size_t to) const {
+    size_t at = 0;
+    for (const Part& p : parts) {
+      const size_t lo = std::max(from, at), hi = std::min(to, at + p.bytes);
+      if (lo < hi) std::memcpy(p.dst + (lo - at), p.src + (lo - at), hi - lo);
+      at += p.bytes;
+    }
+  }
+  void run() const {
+    constexpr size_t kBytesPerThread = 1u << 20;  // about 0.1 ms of copying: several times a thread's start
+    const size_t n = std::min<size_t>({8, (size_t)host_threads(0), total / kBytesPerThread});
+    std::vector<std::thread> threads;
+    size_t done = n > 1 ? total / n : total;  // this thread's share
+    const size_t share = done;
+    size_t from = done;
+    try {
+      for (size_t k = 1; k < n; ++k) {
+        const size_t to = k + 1 == n ? total : from + share;
+        threads.emplace_back([this, from, to] { copy_range(from, to); });
+        from = to;
+      }
+    } catch (...) {  // no more threads to be had: the rest is copied here
+      copy_range(from, total);
+    }
+    copy_range(0, done);
+    for (std::thread& t : threads) t.join();
+  }
+};
+
+// Rows of `width` bytes between pitched buffers: one copy instead of one per row
+// (each costs the host some 5 us, most of a small query's time), as far as the
+// driver's pitch limit of 2^31 - 1 bytes goes.
+void copy_planes(void* dst, size_t dst_pitch, const void* src, size_t src_pitch, size_t width, size_t rows,
+                 cudaMemcpyKind kind, cudaStream_t s) {
+  if (std::max(dst_pitch, src_pitch) <= 0x7fffffffu) {
+    cudaMemcpy2DAsync(dst, dst_pitch, src, src_pitch, width, rows, kind, s);
+    return;
+  }
+  for (size_t r = 0; r < rows; ++r)
+    cudaMemcpyAsync((char*)dst + r * dst_pitch, (const char*)src + r * src_pitch, width, kind, s);
+}
+
 tpt_status ensure_host_staging(tpt_context* ctx, size_t bytes) {
   if (ctx->h_stage_bytes >= bytes) return TPT_OK;
   if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
@@ -86,20 +158,6 @@ tpt_status ensure_host_staging(tpt_context* ctx, size_t bytes) {
   tpt_status st = cuda_check(ctx, cudaMallocHost(&ctx->h_stage, bytes), "cudaMallocHost(staging)");
   if (st) return st;
   ctx->h_stage_bytes = bytes;
-  return TPT_OK;
-}
-
-tpt_status ensure_device_staging(tpt_context* ctx, size_t bytes) {
-  if (ctx->d_stage_bytes >= bytes) return TPT_OK;
-  if (ctx->d_stage) {
-    cudaStreamSynchronize(ctx->stream);
-    cudaFree(ctx->d_stage);
-  }
-  ctx->d_stage = nullptr;
-  ctx->d_stage_bytes = 0;
-  tpt_status st = cuda_check(ctx, cudaMalloc(&ctx->d_stage, bytes), "cudaMalloc(staging)");
-  if (st) return st;
-  ctx->d_stage_bytes = bytes;
   return TPT_OK;
 }
 
@@ -700,6 +758,17 @@ tpt_status tpt_traverse(tpt_context* ctx, const tpt_scene* scene, const float* r
   uint64_t chunk = std::max<uint64_t>(1 << 16, std::min<uint64_t>(1 << 21, (n + 3) / 4));
   struct Out { void* host; const void* dev; size_t planes; };
   const Out outs[4] = {{prim, d_prim, 1}, {t, d_t, 1}, {instance, d_inst, 1}, {bary, d_bary, 3}};
+  // Rays [b, b + m) of every plane, and of one output's planes
+  const size_t pitch = n * 4;
+  auto copy_in_planes = [&](uint64_t b, uint64_t m, const float* src, size_t src_pitch, cudaStream_t s) {
+    copy_planes(d_rays + b, pitch, src, src_pitch, m * 4, in_planes, cudaMemcpyHostToDevice, s);
+  };
+  auto copy_out_planes = [&](uint64_t b, uint64_t m, cudaStream_t s) {
+    for (const Out& o : outs)
+      if (o.host)
+        copy_planes((char*)o.host + b * 4, pitch, (const char*)o.dev + b * 4, pitch, m * 4, o.planes,
+                    cudaMemcpyDeviceToHost, s);
+  };
   if (in_pinned && out_pinned) {
     // Pinned buffers: copies in on one stream, kernels alternating on two
     // streams, copies out on a third, ordered by per-chunk events, so the
@@ -713,8 +782,7 @@ tpt_status tpt_traverse(tpt_context* ctx, const tpt_scene* scene, const float* r
     uint64_t b = 0;
     for (size_t c = 0; c < sizes.size(); ++c) {
       const uint64_t m = sizes[c];
-      for (int p = 0; p < in_planes; ++p)
-        cudaMemcpyAsync(d_rays + p * n + b, rays + p * n + b, m * 4, cudaMemcpyHostToDevice, ctx->copy_in);
+      copy_in_planes(b, m, rays + b, pitch, ctx->copy_in);
       cudaEventRecord(ctx->ev_in[c], ctx->copy_in);
       cudaStream_t s = ctx->pipe[c & 1];
       cudaStreamWaitEvent(s, ctx->ev_in[c], 0);
@@ -724,12 +792,7 @@ tpt_status tpt_traverse(tpt_context* ctx, const tpt_scene* scene, const float* r
       if ((st = cuda_check(ctx, e, "traverse kernel launch"))) return st;
       cudaEventRecord(ctx->ev_done[c], s);
       cudaStreamWaitEvent(ctx->copy_out, ctx->ev_done[c], 0);
-      for (const Out& o : outs) {
-        if (!o.host) continue;
-        for (size_t p = 0; p < o.planes; ++p)
-          cudaMemcpyAsync((char*)o.host + (p * n + b) * 4, (const char*)o.dev + (p * n + b) * 4, m * 4,
-                          cudaMemcpyDeviceToHost, ctx->copy_out);
-      }
+      copy_out_planes(b, m, ctx->copy_out);
       b += m;
     }
     cudaEventRecord(ctx->ev_slot[0], ctx->copy_out);
@@ -737,62 +800,53 @@ tpt_status tpt_traverse(tpt_context* ctx, const tpt_scene* scene, const float* r
     if ((st = cuda_check(ctx, cudaGetLastError(), "traverse pipeline"))) return st;
     return check_device_errors(ctx, ctx->stream);
   }
-  // Pageable buffers: pinned staging slots, pipelined on two streams.
+  // Pageable buffers: pinned staging slots, pipelined on two streams: chunk c is
+  // staged and queued while chunk c - 1 is on the device, and chunk c - 1's
+  // results are drained while chunk c is.
   const uint64_t n_chunks = (n + chunk - 1) / chunk;
-  if (!in_pinned || !out_pinned) {
-    const size_t per_slot = (7 + (size_t)n_out) * chunk * 4;
-    if ((st = ensure_host_staging(ctx, 2 * per_slot))) return st;
-  }
+  const size_t slot_bytes = (7 + (size_t)n_out) * std::min(chunk, n) * 4;
+  if ((st = ensure_host_staging(ctx, 2 * slot_bytes))) return st;
   cudaEventRecord(ctx->ev_start, ctx->stream);
   for (int k = 0; k < 2; ++k) cudaStreamWaitEvent(ctx->pipe[k], ctx->ev_start, 0);
-  for (uint64_t c = 0; c < n_chunks; ++c) {
-    const int k = (int)(c & 1);
-    cudaStream_t s = ctx->pipe[k];
+  auto slot_of = [&](uint64_t c) { return (float*)((char*)ctx->h_stage + (c & 1) * slot_bytes); };
+  auto drain = [&](uint64_t c) {  // results of chunk c from its slot (after the slot's 7 ray planes)
     const uint64_t b = c * chunk, m = std::min<uint64_t>(chunk, n - b);
-    float* hslot = (float*)((char*)ctx->h_stage + k * ((7 + (size_t)n_out) * chunk * 4));
-    if (!in_pinned || !out_pinned) {
-      // the slot is reused every other chunk: wait until its last copy-out is done
-      cudaEventSynchronize(ctx->ev_slot[k]);
-    }
+    cudaEventSynchronize(ctx->ev_slot[c & 1]);
+    HostCopies copies;
+    const float* src = slot_of(c) + 7 * m;
+    for (const Out& o : outs)
+      if (o.host)
+        for (size_t p = 0; p < o.planes; ++p, src += m) copies.add((char*)o.host + (p * n + b) * 4, src, m * 4);
+    copies.run();
+  };
+  for (uint64_t c = 0; c < n_chunks; ++c) {
+    cudaStream_t s = ctx->pipe[c & 1];
+    const uint64_t b = c * chunk, m = std::min<uint64_t>(chunk, n - b);
+    float* hslot = slot_of(c);
     if (in_pinned) {
-      for (int p = 0; p < in_planes; ++p)
-        cudaMemcpyAsync(d_rays + p * n + b, rays + p * n + b, m * 4, cudaMemcpyHostToDevice, s);
+      copy_in_planes(b, m, rays + b, pitch, s);
     } else {
-      for (int p = 0; p < in_planes; ++p) std::memcpy(hslot + p * m, rays + p * n + b, m * 4);
-      for (int p = 0; p < in_planes; ++p)
-        cudaMemcpyAsync(d_rays + p * n + b, hslot + p * m, m * 4, cudaMemcpyHostToDevice, s);
+      // the slot's last chunk but one has been drained (or, with pinned results,
+      // its event tells when its rays have been read)
+      if (out_pinned && c >= 2) cudaEventSynchronize(ctx->ev_slot[c & 1]);
+      HostCopies copies;
+      for (int p = 0; p < in_planes; ++p) copies.add(hslot + p * m, rays + p * n + b, m * 4);
+      copies.run();
+      copy_in_planes(b, m, hslot, m * 4, s);
     }
     // the kernel reads plane p of the chunk at d_rays + p*n + b: pass a view with stride n
     cudaError_t e = launch_traverse_strided(scene->geo, d_rays + b, n, m, mode, d_prim + b, d_t + b,
                                             d_inst ? d_inst + b : nullptr, d_bary ? d_bary + b : nullptr, n,
                                             next_counter(ctx), ctx->d_err, ctx->num_sms, s, nullptr, nullptr);
     if ((st = cuda_check(ctx, e, "traverse kernel launch"))) return st;
-    float* hout = hslot + 7 * m;
-    size_t ho = 0;
-    for (const Out& o : outs) {
-      if (!o.host) continue;
-      for (size_t p = 0; p < o.planes; ++p) {
-        const char* src = (const char*)o.dev + (p * n + b) * 4;
-        if (out_pinned) {
-          cudaMemcpyAsync((char*)o.host + (p * n + b) * 4, src, m * 4, cudaMemcpyDeviceToHost, s);
-        } else {
-          cudaMemcpyAsync(hout + ho * m, src, m * 4, cudaMemcpyDeviceToHost, s);
-          ++ho;
-        }
-      }
-    }
-    if (!out_pinned) {
-      // drain the slot before it is reused (two chunks later)
-      cudaStreamSynchronize(s);
-      size_t h2 = 0;
-      for (const Out& o : outs) {
-        if (!o.host) continue;
-        for (size_t p = 0; p < o.planes; ++p, ++h2)
-          std::memcpy((char*)o.host + (p * n + b) * 4, hout + h2 * m, m * 4);
-      }
-    }
-    cudaEventRecord(ctx->ev_slot[k], s);
+    if (out_pinned)
+      copy_out_planes(b, m, s);
+    else  // the outputs' planes follow one another on the device
+      copy_planes(hslot + 7 * m, m * 4, d_prim + b, pitch, m * 4, n_out, cudaMemcpyDeviceToHost, s);
+    cudaEventRecord(ctx->ev_slot[c & 1], s);
+    if (!out_pinned && c >= 1) drain(c - 1);
   }
+  if (!out_pinned) drain(n_chunks - 1);
   for (int k = 0; k < 2; ++k) {
     cudaEventRecord(ctx->ev_slot[k], ctx->pipe[k]);
     cudaStreamWaitEvent(ctx->stream, ctx->ev_slot[k], 0);

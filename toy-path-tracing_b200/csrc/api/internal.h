@@ -130,6 +130,9 @@ tpt_status cuda_check(tpt_context* ctx, cudaError_t e, const char* what);
 tpt_status check_device_errors(tpt_context* ctx, cudaStream_t stream);
 // Records that entry point `name` queued device work whose checks are read later.
 void note_device_call(tpt_context* ctx, const char* name);
+// Grows the context's device staging buffer (ctx->d_stage), which host-buffer
+// calls use and have finished with when they return.
+tpt_status ensure_device_staging(tpt_context* ctx, size_t bytes);
 // cudaSetDevice(ctx->device) with its status checked.
 tpt_status set_device(tpt_context* ctx);
 

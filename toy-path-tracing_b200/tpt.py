@@ -98,17 +98,36 @@ class OpenPbrDesc(C.Structure):
 assert C.sizeof(OpenPbrDesc) == 45 * 4
 
 
-def openpbr_desc(m: dict) -> OpenPbrDesc:
-    """A tpt_openpbr_desc from a material dict (missing keys: defaults)."""
+def _set_openpbr_field(d: OpenPbrDesc, name: str, k: int, v):
+    if k == 3:
+        if not (type(v) is np.ndarray and v.shape == (3,)):
+            v = np.broadcast_to(np.asarray(v, np.float32), (3,))
+        getattr(d, name)[:] = v.astype(np.float32).tolist()
+    elif name == "geometry_thin_walled":
+        setattr(d, name, int(v))
+    else:
+        setattr(d, name, float(np.float32(v)))
+
+
+def _default_openpbr_desc() -> OpenPbrDesc:
     d = OpenPbrDesc()
     for name, k, default in OPENPBR_FIELDS:
-        v = m.get(name, default)
-        if k == 3:
-            getattr(d, name)[:] = [float(np.float32(x)) for x in np.broadcast_to(np.asarray(v, np.float32), (3,))]
-        elif name == "geometry_thin_walled":
-            setattr(d, name, int(v))
-        else:
-            setattr(d, name, float(np.float32(v)))
+        _set_openpbr_field(d, name, k, default)
+    return d
+
+
+_OPENPBR_DEFAULT = _default_openpbr_desc()
+_OPENPBR_WIDTH = {name: k for name, k, _ in OPENPBR_FIELDS}
+
+
+def openpbr_desc(m: dict) -> OpenPbrDesc:
+    """A tpt_openpbr_desc from a material dict (missing keys: defaults)."""
+    # only the keys given are converted (a material with five of the 31 fields: 4 us instead of 49)
+    d = OpenPbrDesc.from_buffer_copy(_OPENPBR_DEFAULT)
+    for name, v in m.items():
+        k = _OPENPBR_WIDTH.get(name)
+        if k is not None:
+            _set_openpbr_field(d, name, k, v)
     return d
 
 
