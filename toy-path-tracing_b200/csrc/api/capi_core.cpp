@@ -138,7 +138,7 @@ struct HostCopies {
 };
 
 // Rows of `width` bytes between pitched buffers: one copy instead of one per row
-// (each costs the host some 5 us, most of a small query's time), as far as the
+// (each costs the host some 3 us, a quarter of a small query's time), as far as the
 // driver's pitch limit of 2^31 - 1 bytes goes.
 void copy_planes(void* dst, size_t dst_pitch, const void* src, size_t src_pitch, size_t width, size_t rows,
                  cudaMemcpyKind kind, cudaStream_t s) {

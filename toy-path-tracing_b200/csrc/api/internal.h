@@ -264,6 +264,13 @@ cudaError_t launch_bsdf_sample(const DevRenderData& rd, uint32_t material, uint6
                                cudaStream_t s);
 
 // scene_render_upload.cpp: materials, shading arrays, light tree, emitter map.
+// Device gather of the shading records (scene_bake.cu): mesh m's triangles start
+// at tri_base of the concatenated index array, its vertices at vtx_base.
+struct MeshSpan {
+  uint32_t vtx_base, tri_base;
+};
+cudaError_t launch_bake_shade_tris(const MeshSpan* meshes, uint32_t n_meshes, const float* pos, const float* nrm,
+                                   const float* uv, const uint32_t* idx, uint64_t n, DevShadeTri* out, cudaStream_t s);
 tpt_status upload_render_data(tpt_scene* s, const tpt_scene_desc* desc);
 // One OpenPBR material lowered for the device (make_bsdf's material part),
 // building the tables it reads on first use.

@@ -2,6 +2,7 @@
 // shading records, the SG light tree and the emitter-triangle -> leaf map that
 // replaces the reference's HashMap / linear searches (light_tree/mod.rs:101-108,
 // scene/mod.rs:583-594).
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -52,6 +53,53 @@ tpt_status put(tpt_scene* s, const std::vector<T>& v, const T** dst) {
   }
   *dst = (const T*)p;
   return TPT_OK;
+}
+
+// Device memory of one call.
+struct TempArrays {
+  tpt_context* ctx;
+  std::vector<void*> ptrs;
+  explicit TempArrays(tpt_context* c) : ctx(c) {}
+  ~TempArrays() {
+    for (void* p : ptrs) cudaFree(p);
+  }
+  template <class T>
+  tpt_status put(const std::vector<T>& v, const T** dst) {
+    void* p = nullptr;
+    tpt_status st = cuda_check(ctx, cudaMalloc(&p, std::max<size_t>(v.size() * sizeof(T), 16)), "cudaMalloc(upload)");
+    if (st) return st;
+    ptrs.push_back(p);
+    *dst = (const T*)p;
+    return cuda_check(ctx, cudaMemcpy(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice), "cudaMemcpy(upload)");
+  }
+};
+
+// The shading records: the vertex arrays go to the device as they are (a fifth
+// of the records' size for a closed mesh) and are gathered there.
+tpt_status put_shade_tris(tpt_scene* s, const std::vector<MeshSpan>& spans, const std::vector<float>& pos,
+                          const std::vector<float>& nrm, const std::vector<float>& uv,
+                          const std::vector<uint32_t>& idx, const DevShadeTri** dst) {
+  TempArrays tmp(s->ctx);
+  const MeshSpan* d_spans = nullptr;
+  const float *d_pos = nullptr, *d_nrm = nullptr, *d_uv = nullptr;
+  const uint32_t* d_idx = nullptr;
+  void* out = nullptr;
+  const uint64_t n = idx.size() / 3;
+  tpt_status st = scene_alloc(s, n * sizeof(DevShadeTri), &out);
+  if (!st) st = tmp.put(spans, &d_spans);
+  if (!st) st = tmp.put(pos, &d_pos);
+  if (!st) st = tmp.put(nrm, &d_nrm);
+  if (!st) st = tmp.put(uv, &d_uv);
+  if (!st) st = tmp.put(idx, &d_idx);
+  if (st) return st;
+  cudaStream_t stream = s->ctx->stream;
+  st = cuda_check(s->ctx,
+                  launch_bake_shade_tris(d_spans, (uint32_t)spans.size(), d_pos, d_nrm, d_uv, d_idx, n,
+                                         (DevShadeTri*)out, stream),
+                  "shading record launch");
+  if (!st) st = cuda_check(s->ctx, cudaStreamSynchronize(stream), "shading records");
+  *dst = (const DevShadeTri*)out;
+  return st;
 }
 }  // namespace
 
@@ -130,23 +178,20 @@ tpt_status upload_render_data(tpt_scene* s, const tpt_scene_desc* desc) {
   // vertex attributes, concatenated per mesh
   std::vector<float> pos, nrm, uv;
   std::vector<uint32_t> idx;
-  std::vector<DevMeshInfo> minfo(desc->num_meshes);
+  std::vector<MeshSpan> spans(desc->num_meshes);
   std::vector<HostMesh> hmesh(desc->num_meshes);
   for (uint32_t m = 0; m < desc->num_meshes; ++m) {
     const tpt_mesh_desc& md = desc->meshes[m];
-    DevMeshInfo mi{};
-    mi.vtx_base = (uint32_t)(pos.size() / 3);
-    mi.idx_base = (uint32_t)idx.size();
-    mi.num_tris = (uint32_t)(md.num_indices / 3);
-    mi.flags = (md.normals ? 1u : 0u) | (md.uvs ? 2u : 0u);
+    const MeshSpan mi{(uint32_t)(pos.size() / 3), (uint32_t)(idx.size() / 3)};
     pos.insert(pos.end(), md.positions, md.positions + 3 * md.num_vertices);
     if (md.normals) nrm.resize(pos.size(), 0.0f), std::memcpy(&nrm[3 * mi.vtx_base], md.normals, 12 * md.num_vertices);
     else nrm.resize(pos.size(), 0.0f);
     uv.resize(2 * (pos.size() / 3), 0.0f);
     if (md.uvs) std::memcpy(&uv[2 * mi.vtx_base], md.uvs, 8 * md.num_vertices);
     idx.insert(idx.end(), md.indices, md.indices + md.num_indices);
-    minfo[m] = mi;
-    hmesh[m] = HostMesh{md.positions, md.normals, md.uvs, md.indices, (uint32_t)md.num_vertices, mi.num_tris};
+    spans[m] = mi;
+    hmesh[m] = HostMesh{md.positions, md.normals, md.uvs, md.indices, (uint32_t)md.num_vertices,
+                        (uint32_t)(md.num_indices / 3)};
   }
 
   // point, spot and directional lights (PointLight::new, SpotLight::new, DirectionalLight::new)
@@ -219,7 +264,7 @@ tpt_status upload_render_data(tpt_scene* s, const tpt_scene_desc* desc) {
           return set_error(ctx, TPT_ERR_INVALID_ARG, "light tree leaf names an unknown point or spot light");
       } else if (leaf) {
         if (n.leaf_instance >= desc->num_instances ||
-            n.leaf_triangle >= minfo[desc->instances[n.leaf_instance].mesh_index].num_tris)
+            n.leaf_triangle >= hmesh[desc->instances[n.leaf_instance].mesh_index].num_triangles)
           return set_error(ctx, TPT_ERR_INVALID_ARG, "light tree leaf names an unknown triangle");
       } else if (n.left >= nn || n.right >= nn) {
         return set_error(ctx, TPT_ERR_INVALID_ARG, "light tree child index out of range");
@@ -243,12 +288,12 @@ tpt_status upload_render_data(tpt_scene* s, const tpt_scene_desc* desc) {
     const float cols[12] = {w[0], w[1], w[2], w[4], w[5], w[6], w[8], w[9], w[10], w[12], w[13], w[14]};
     std::memcpy(d.l2w, cols, sizeof cols);
     std::memcpy(d.n2w, id.normal_to_world, 36);
-    d.mesh = id.mesh_index;
+    d.tri_base = spans[id.mesh_index].tri_base;
     d.material = id.material_index;
     d.leaf_base = kInvalidNode;
     if (desc->num_materials && hmats[id.material_index].may_emit()) {
       d.leaf_base = map_size;
-      map_size += minfo[id.mesh_index].num_tris;
+      map_size += hmesh[id.mesh_index].num_triangles;
     }
     sinst[i] = d;
   }
@@ -280,11 +325,7 @@ tpt_status upload_render_data(tpt_scene* s, const tpt_scene_desc* desc) {
   DevRenderData& R = s->render;
   tpt_status st = TPT_OK;
   if (!st) st = put(s, sinst, &R.inst);
-  if (!st) st = put(s, minfo, &R.meshes);
-  if (!st) st = put(s, pos, &R.pos);
-  if (!st) st = put(s, nrm, &R.nrm);
-  if (!st) st = put(s, uv, &R.uv);
-  if (!st) st = put(s, idx, &R.idx);
+  if (!st) st = put_shade_tris(s, spans, pos, nrm, uv, idx, &R.tris);
   if (!st) st = put(s, dmats, &R.mats);
   if (!st) st = put(s, lnodes, &R.ltree);
   if (!st) st = put(s, emap, &R.emitter_leaf);

@@ -65,30 +65,24 @@ struct TriData {
 
 __device__ __forceinline__ void fetch_triangle(const DevRender& S, uint32_t inst, uint32_t tri, TriData& T,
                                                bool want_shading) {
-  const DevShadeInstance* I = S.d.inst + inst;
-  const DevMeshInfo M = S.d.meshes[__ldg(&I->mesh)];
-  float l2w[12];
+  const float* I = S.d.inst[inst].l2w;
+  float iw[24], tw[24];  // the records' first 96 bytes
+  ldg32(I, *reinterpret_cast<float(*)[8]>(iw));
+  ldg32(I + 8, *reinterpret_cast<float(*)[8]>(iw + 8));
+  if (want_shading) ldg32(I + 16, *reinterpret_cast<float(*)[8]>(iw + 16));
+  const float* R = S.d.tris[__float_as_uint(iw[12]) + tri].p;
+  ldg32(R, *reinterpret_cast<float(*)[8]>(tw));
+  ldg32(R + 8, *reinterpret_cast<float(*)[8]>(tw + 8));
+  if (want_shading) ldg32(R + 16, *reinterpret_cast<float(*)[8]>(tw + 16));
 #pragma unroll
-  for (int k = 0; k < 12; ++k) l2w[k] = __ldg(&I->l2w[k]);
-  uint32_t vi[3];
-#pragma unroll
-  for (int k = 0; k < 3; ++k) vi[k] = M.vtx_base + __ldg(S.d.idx + M.idx_base + 3 * tri + k);
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    const V3 lp = V3{__ldg(S.d.pos + 3 * vi[k]), __ldg(S.d.pos + 3 * vi[k] + 1), __ldg(S.d.pos + 3 * vi[k] + 2)};
-    T.p[k] = xform_point(l2w, lp);
-  }
+  for (int k = 0; k < 3; ++k) T.p[k] = xform_point(iw, V3{tw[3 * k], tw[3 * k + 1], tw[3 * k + 2]});
   if (!want_shading) return;
-  float n2w[9];
-#pragma unroll
-  for (int k = 0; k < 9; ++k) n2w[k] = __ldg(&I->n2w[k]);
+  const float* n2w = iw + 13;
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    V3 ln = V3{0.0f, 0.0f, 0.0f};
-    if (M.flags & 1u) ln = V3{__ldg(S.d.nrm + 3 * vi[k]), __ldg(S.d.nrm + 3 * vi[k] + 1), __ldg(S.d.nrm + 3 * vi[k] + 2)};
-    T.n[k] = normalize_or_zero(mat3_mul(n2w, ln));
-    T.u[k] = (M.flags & 2u) ? __ldg(S.d.uv + 2 * vi[k]) : 0.0f;
-    T.v[k] = (M.flags & 2u) ? __ldg(S.d.uv + 2 * vi[k] + 1) : 0.0f;
+    T.n[k] = normalize_or_zero(mat3_mul(n2w, V3{tw[9 + 3 * k], tw[10 + 3 * k], tw[11 + 3 * k]}));
+    T.u[k] = tw[18 + 2 * k];
+    T.v[k] = tw[19 + 2 * k];
   }
 }
 

@@ -113,15 +113,25 @@ struct alignas(16) DevOpenPbr {
   uint32_t pad2[2];
 };
 
-struct alignas(16) DevShadeInstance {
+// What shading reads of an instance, in three 32-byte loads (two for positions).
+struct alignas(32) DevShadeInstance {
   float l2w[12];  // local_to_world affine columns c0..c3 (xyz each)
+  uint32_t tri_base;   // first DevShadeTri of the mesh
   float n2w[9];   // normal_to_world, column-major
-  uint32_t mesh;
   uint32_t material;
   uint32_t leaf_base;  // first emitter-map slot of this instance, or 0xFFFFFFFF
   uint32_t pad[8];
 };
 static_assert(sizeof(DevShadeInstance) == 128, "shade instance record");
+
+// A triangle's vertices in mesh space, in mesh order (zeros for attributes the
+// mesh does not have).  A record per triangle instead of indices and vertex
+// arrays: a hit reads three 32-byte loads, one load away from its instance,
+// instead of 27 single words two loads away (mesh, then indices).
+struct alignas(32) DevShadeTri {
+  float p[9], n[9], uv[6];
+};
+static_assert(sizeof(DevShadeTri) == 96, "shade triangle record");
 
 // Scene::area_light_triangles entry (scene/mod.rs:48-54): emissive triangle,
 // its area, selection weight (area * max_emission) and the running prefix.
@@ -172,17 +182,9 @@ struct DevEnvironment {
   DevEnvDist mis;        // MIS-compensated: (luminance - mean) x sin(theta) where above epsilon
 };
 
-struct DevMeshInfo {
-  uint32_t vtx_base, idx_base, num_tris, flags;  // flags bit 0: normals, bit 1: uvs
-};
-
 struct DevRenderData {
   const DevShadeInstance* inst;
-  const DevMeshInfo* meshes;
-  const float* pos;
-  const float* nrm;
-  const float* uv;
-  const uint32_t* idx;
+  const DevShadeTri* tris;
   const DevMaterialRec* mats;
   const DevLightNodeRec* ltree;
   const uint32_t* emitter_leaf;
