@@ -44,7 +44,7 @@ struct __align__(32) DevTriPair {  // triangles 2k and 2k + 1 of the concatenate
 };
 static_assert(sizeof(DevTriPair) == 96, "triangle pair record");
 
-struct __align__(16) DevInstance {
+struct __align__(32) DevInstance {
   float4 m0;  // c0.x c0.y c0.z c1.x
   float4 m1;  // c1.y c1.z c2.x c2.y
   float4 m2;  // c2.z c3.x c3.y c3.z

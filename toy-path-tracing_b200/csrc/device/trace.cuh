@@ -43,6 +43,7 @@ struct RayPre {
   int kz;               // axis of the largest |d| component; x, y follow it cyclically
   bool exact;           // an infinite reciprocal lane: use select min/max
   bool no_tri;          // permuted d.z == 0: no triangle can be hit
+  bool tris_ready;      // sx, sy, sz, kz and no_tri are set; before, (sx, sy, sz) is the direction
 };
 
 // (kx, ky, kz) components, kx = kz + 1 and ky = kz + 2 modulo 3
@@ -52,29 +53,29 @@ __device__ __forceinline__ void permute3(float x, float y, float z, int kz, floa
   pz = kz == 0 ? x : (kz == 1 ? y : z);
 }
 
-__device__ __forceinline__ void ray_setup(RayPre& r, float ox, float oy, float oz, float dx, float dy, float dz) {
-  r.ox = ox; r.oy = oy; r.oz = oz;
+// A ray's setup comes in two parts, each made where it is first read: the
+// reciprocals for box tests (an instance whose tree is a single leaf has none, and
+// the world ray needs them back only for a TLAS node), and the permutation and
+// shear for triangle tests (most instances a ray enters show it no leaf).  Each
+// part is three divisions.
+__device__ __forceinline__ void ray_setup_boxes(RayPre& r, float dx, float dy, float dz) {
   r.ix = safe_inv(dx); r.iy = safe_inv(dy); r.iz = safe_inv(dz);
   // NaN can only come from 0 * inf in (b - o) * inv, i.e. from a reciprocal
   // lane that is infinite (or zero, for an infinite direction component).
   r.exact = !(isfinite(r.ix) && isfinite(r.iy) && isfinite(r.iz) && r.ix != 0.0f && r.iy != 0.0f && r.iz != 0.0f);
-  float ax = fabsf(dx), ay = fabsf(dy), az = fabsf(dz);
-  int kz = (ax > ay) ? (ax > az ? 0 : 2) : (ay > az ? 1 : 2);  // math/mod.rs:148-156
-  r.kz = kz;
+}
+// The direction waits in (sx, sy, sz) until then.
+__device__ __forceinline__ void ray_setup_tris(RayPre& r) {
+  const float dx = r.sx, dy = r.sy, dz = r.sz;
+  const float ax = fabsf(dx), ay = fabsf(dy), az = fabsf(dz);
+  r.kz = (ax > ay) ? (ax > az ? 0 : 2) : (ay > az ? 1 : 2);  // math/mod.rs:148-156
   float pdx, pdy, pdz;
-  permute3(dx, dy, dz, kz, pdx, pdy, pdz);
+  permute3(dx, dy, dz, r.kz, pdx, pdy, pdz);
   r.no_tri = (pdz == 0.0f);
   r.sx = -pdx / pdz;
   r.sy = -pdy / pdz;
-  r.sz = kz == 0 ? r.ix : (kz == 1 ? r.iy : r.iz);  // 1 / pdz (a zero pdz hits no triangle)
-}
-
-// The part of ray_setup that box tests read: at the TLAS no triangle is tested.
-__device__ __forceinline__ void ray_setup_boxes(RayPre& r, float ox, float oy, float oz, float dx, float dy,
-                                                float dz) {
-  r.ox = ox; r.oy = oy; r.oz = oz;
-  r.ix = safe_inv(dx); r.iy = safe_inv(dy); r.iz = safe_inv(dz);
-  r.exact = !(isfinite(r.ix) && isfinite(r.iy) && isfinite(r.iz) && r.ix != 0.0f && r.iy != 0.0f && r.iz != 0.0f);
+  r.sz = 1.0f / pdz;
+  r.tris_ready = true;
 }
 
 __device__ __forceinline__ float dop(float a, float b, float c, float d) {
@@ -272,6 +273,7 @@ struct TravState {
   uint32_t next;
   int sp, floor_sp;
   bool in_blas;
+  bool boxes_ready;                    // the current level's ray is set up for box tests
   uint32_t node_base;                  // first node of the current level (TLAS or BLAS)
   uint32_t tri_base, inst_id;
   // ALPHA instantiations only
@@ -302,8 +304,11 @@ __device__ __forceinline__ void enter_instance(const DevGeometry& G, TravState& 
   s.inst_id = id;
   if (ALPHA) s.alpha = s.alpha_on ? __ldg(G.inst_alpha + id) : 1.0f;
   const DevInstance* I = G.instances + id;
-  const float4 m0 = __ldg(&I->m0), m1 = __ldg(&I->m1), m2 = __ldg(&I->m2);
-  const uint4 meta = __ldg(reinterpret_cast<const uint4*>(&I->node_base));
+  float q0[8], q1[8];
+  ldg32(&I->m0, q0);
+  ldg32(&I->m2, q1);
+  const float4 m0 = make_float4(q0[0], q0[1], q0[2], q0[3]), m1 = make_float4(q0[4], q0[5], q0[6], q0[7]);
+  const float4 m2 = make_float4(q1[0], q1[1], q1[2], q1[3]);
   const float ox = s.wox, oy = s.woy, oz = s.woz, dx = s.wdx, dy = s.wdy, dz = s.wdz;
   float lox = m0.x * ox, loy = m0.y * ox, loz = m0.z * ox;
   lox = m0.w * oy + lox; loy = m1.x * oy + loy; loz = m1.y * oy + loz;
@@ -312,12 +317,16 @@ __device__ __forceinline__ void enter_instance(const DevGeometry& G, TravState& 
   float ldx = m0.x * dx, ldy = m0.y * dx, ldz = m0.z * dx;
   ldx = m0.w * dy + ldx; ldy = m1.x * dy + ldy; ldz = m1.y * dy + ldz;
   ldx = m1.z * dz + ldx; ldy = m1.w * dz + ldy; ldz = m2.x * dz + ldz;
-  ray_setup(s.r, lox, loy, loz, ldx, ldy, ldz);
-  s.node_base = meta.x;
-  s.tri_base = meta.y;
+  s.r.ox = lox; s.r.oy = loy; s.r.oz = loz;
+  s.r.sx = ldx; s.r.sy = ldy; s.r.sz = ldz;
+  s.r.tris_ready = false;
+  s.node_base = __float_as_uint(q1[4]);
+  s.tri_base = __float_as_uint(q1[5]);
   s.in_blas = true;
   s.floor_sp = s.sp;
-  s.next = meta.z;
+  s.next = __float_as_uint(q1[6]);
+  s.boxes_ready = !(s.next & kLeafBit);
+  if (s.boxes_ready) ray_setup_boxes(s.r, ldx, ldy, ldz);
 }
 
 template <class Stack>
@@ -330,9 +339,14 @@ __device__ __forceinline__ void trav_pop(const DevGeometry& G, TravState& s, Sta
     // the instance's BLAS is done: back to the TLAS with the world ray
     s.in_blas = false;
     s.node_base = G.tlas_node_base;
-    ray_setup_boxes(s.r, s.wox, s.woy, s.woz, s.wdx, s.wdy, s.wdz);
+    s.boxes_ready = false;
   }
   s.next = st.get(--s.sp);
+  if (!s.boxes_ready && !(s.next & kLeafBit)) {  // a TLAS node after an instance
+    s.r.ox = s.wox; s.r.oy = s.woy; s.r.oz = s.woz;
+    ray_setup_boxes(s.r, s.wdx, s.wdy, s.wdz);
+    s.boxes_ready = true;
+  }
 }
 
 // ALPHA: the caller has AuxRng states (aux: the ray's, NULL = none), which the
@@ -362,7 +376,9 @@ __device__ __forceinline__ void trav_init(const DevGeometry& G, TravState& s, fl
     // TLAS is a single-instance root leaf (qbvh.rs:615-620): go straight to it
     enter_instance<ALPHA>(G, s, __ldg(G.tlas_prims + (root & 0xFFFFFFu)));
   } else {
-    ray_setup_boxes(s.r, ox, oy, oz, dx, dy, dz);
+    s.r.ox = ox; s.r.oy = oy; s.r.oz = oz;
+    ray_setup_boxes(s.r, dx, dy, dz);
+    s.boxes_ready = true;
     s.next = root;
   }
 }
@@ -435,6 +451,7 @@ __device__ __forceinline__ void leaf_step(const DevGeometry& G, TravState& s, St
   const uint32_t count = (w >> 24) & 0x7Fu, off = w & 0xFFFFFFu;
   if (s.in_blas) {
     // BLAS leaf: triangles in leaf order, t_max shrinking on each hit
+    if (!s.r.tris_ready) ray_setup_tris(s.r);
     uint32_t g = s.tri_base + off;
     for (const uint32_t end = g + count; g != end; ++g) {
       const DevTri tri = load_tri(G.tris, g);

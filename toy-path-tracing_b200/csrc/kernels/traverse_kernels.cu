@@ -35,6 +35,8 @@ constexpr int kMinBlocks = 7;
 // triangle instanced scene / 2^22 rays in the Cornell box, ms): 16-byte loads
 // and branches 8.15 / 5.70 / 3.11; this kernel with kNodeMin 0 5.94 / 4.61 / 2.44,
 // 8 5.88 / 3.66 / 2.10, 11 5.92 / 3.69 / 2.01.  kRefillMin 8 or 16: 4 % and 1 % slower.
+// With ray setups made on first use 8 gives 5.88 / 3.52 / 1.88, 13 5.87 / 3.57 / 1.78
+// and, in renders of the instanced scene, 1-2 % more time than 8.
 constexpr int kRefillMin = 12;
 constexpr int kNodeMin = 8;
 
