@@ -6,7 +6,7 @@
 // sample within a job).  It is cut into chunks of at most the wavefront
 // capacity, on pixel boundaries so that each pixel's samples are accumulated
 // in order within one chunk.  Each chunk runs generate -> (traverse -> shade
-// -> shadow traverse -> resolve) x (deepest job in the chunk + 1) -> finalize,
+// -> shadow traverse -> resolve) x (deepest job in the chunk + 1),
 // with every stage reading each slot's job record, then one accumulate launch
 // per job segment of the chunk.
 #include <algorithm>
@@ -106,7 +106,6 @@ tpt_status render_batch(tpt_context* ctx, const tpt_render_job* jobs, int n_jobs
     return set_error(ctx, TPT_ERR_CAPACITY, "a pixel's spp exceeds the wavefront capacity of the batch");
   tpt_status st = ensure_jobs(ctx, n_jobs);
   if (!st) st = ensure_wavefront(ctx, capacity);
-  if (!st) st = ensure_scratch(ctx, (size_t)capacity * 12);
   if (st) return st;
   if ((st = cuda_check(ctx, cudaMemcpyAsync(ctx->d_jobs, dj.data(), n_jobs * sizeof(DevJob), cudaMemcpyHostToDevice, s),
                        "upload job table")))
@@ -114,7 +113,6 @@ tpt_status render_batch(tpt_context* ctx, const tpt_render_job* jobs, int n_jobs
   bool alpha = false;
   for (int j = 0; j < n_jobs; ++j) alpha = alpha || jobs[j].scene->geo.inst_alpha != nullptr;
   const WfBuffers B = wavefront_view(ctx->wf, alpha);
-  float* samples = (float*)ctx->d_scratch;
   const DevGeometry no_geo{};
   bool lights = false;
   for (int j = 0; j < n_jobs; ++j) lights = lights || jobs[j].scene->render.num_extra_lights > 0;
@@ -123,10 +121,9 @@ tpt_status render_batch(tpt_context* ctx, const tpt_render_job* jobs, int n_jobs
     for (uint32_t b = 0; e == cudaSuccess && b <= c.max_depth; ++b)
       e = enqueue_bounce(ctx, s, no_geo, DevRenderData{}, RenderLaunch{}, B, ctx->d_jobs, (int)(b & 1u), b > 0,
                          lights);
-    if (e == cudaSuccess) e = launch_wf_finalize(B, c.n_paths, samples, s);
     for (const Segment& g : c.segs) {
       if (e != cudaSuccess) break;
-      e = launch_accumulate(samples + 3 * g.sample_offset, L[g.job].spp, g.p0, g.n, L[g.job].cam.exposure,
+      e = launch_wf_accumulate(B, (uint32_t)g.sample_offset, L[g.job].spp, g.p0, g.n, L[g.job].cam.exposure,
                             out_rgb[g.job], s);
     }
     if ((st = cuda_check(ctx, e, "batched wavefront launch"))) return st;

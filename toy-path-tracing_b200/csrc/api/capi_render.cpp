@@ -158,7 +158,7 @@ tpt_status ensure_wavefront(tpt_context* ctx, uint32_t capacity) {
 }
 
 // Paths [first, first + n) through the wavefront stages; radiance per path into
-// samples.  With A, the adjoint replay instead: samples holds the paths'
+// samples (NULL: it stays in the arena's planes).  With A, the adjoint replay instead: samples holds the paths'
 // radiance from a forward pass and the gradients go to A->grad.
 tpt_status render_wavefront(tpt_context* ctx, const tpt_render_job* job, const RenderLaunch& L, uint64_t first,
                             uint32_t n, float* samples, cudaStream_t s, const DevAdjoint* A) {
@@ -203,7 +203,7 @@ tpt_status render_wavefront(tpt_context* ctx, const tpt_render_job* job, const R
     if (e == cudaSuccess) e = cudaMemsetAsync(B.counts + 2, 0, 4, s);
     if (e == cudaSuccess) e = launch_wf_shade(geo, rd, L, B, cur, s, A);
   }
-  if (e == cudaSuccess && !A) e = launch_wf_finalize(B, n, samples, s);
+  if (e == cudaSuccess && !A && samples) e = launch_wf_finalize(B, n, samples, s);
   return cuda_check(ctx, e, "wavefront launch");
 }
 
@@ -397,19 +397,24 @@ tpt_status tpt_render_pixels_device(tpt_context* ctx, const tpt_render_job* job,
   note_device_call(ctx, first_pixel == 0 && num_pixels == total ? "tpt_render_device" : "tpt_render_pixels_device");
   const uint32_t pix_begin = (uint32_t)first_pixel, pix_end = (uint32_t)(first_pixel + num_pixels);
   const uint32_t cp = chunk_pixels(L, ctx->batch_capacity);
-  if ((st = ensure_scratch(ctx, (size_t)cp * L.spp * 12))) return st;
-  float* samples = (float*)ctx->d_scratch;
   const uint32_t exec = job->execution == TPT_EXEC_AUTO ? ctx->tuned_execution : job->execution;
+  const bool wavefront = exec != TPT_EXEC_MEGAKERNEL && job->integrator != TPT_INTEGRATOR_BDPT;
+  if (!wavefront && (st = ensure_scratch(ctx, (size_t)cp * L.spp * 12))) return st;
+  float* samples = (float*)ctx->d_scratch;
   for (uint32_t p0 = pix_begin; p0 < pix_end; p0 += cp) {
     const uint32_t n = std::min(cp, pix_end - p0);
-    if (job->integrator == TPT_INTEGRATOR_BDPT && exec != TPT_EXEC_MEGAKERNEL) {
+    if (wavefront) {  // straight from the arena's radiance planes
+      if ((st = render_wavefront(ctx, job, L, (uint64_t)p0 * L.spp, n * L.spp, nullptr, s))) return st;
+      cudaError_t e = launch_wf_accumulate(ctx->wf, 0, L.spp, p0 - pix_begin, n, L.cam.exposure, out_rgb, s);
+      if ((st = cuda_check(ctx, e, "accumulate kernel launch"))) return st;
+      continue;
+    }
+    if (exec != TPT_EXEC_MEGAKERNEL) {
       if ((st = render_bdpt_wavefront(ctx, job, L, (uint64_t)p0 * L.spp, (uint64_t)n * L.spp, samples, s))) return st;
-    } else if (exec == TPT_EXEC_MEGAKERNEL || job->integrator == TPT_INTEGRATOR_BDPT) {
+    } else {
       cudaError_t e = launch_render(job->scene->geo, job->scene->render, L, samples, (uint64_t)p0 * L.spp,
                                     (uint64_t)n * L.spp, ctx->d_err, ctx->num_sms, s, next_counter(ctx));
       if ((st = cuda_check(ctx, e, "render kernel launch"))) return st;
-    } else {
-      if ((st = render_wavefront(ctx, job, L, (uint64_t)p0 * L.spp, n * L.spp, samples, s))) return st;
     }
     cudaError_t e = launch_accumulate(samples, L.spp, p0 - pix_begin, n, L.cam.exposure, out_rgb, s);
     if ((st = cuda_check(ctx, e, "accumulate kernel launch"))) return st;

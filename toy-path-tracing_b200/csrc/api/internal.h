@@ -223,6 +223,8 @@ cudaError_t launch_wf_generate_batch(const DevJob* jobs, uint32_t n_jobs, const 
 cudaError_t launch_wf_shade_batch(const DevJob* jobs, const WfBuffers& B, int cur, cudaStream_t s, int block,
                                   bool lights);
 cudaError_t launch_wf_finalize(const WfBuffers& B, uint32_t n_paths, float* samples, cudaStream_t s);
+cudaError_t launch_wf_accumulate(const WfBuffers& B, uint32_t first_slot, uint32_t spp, uint32_t first_pixel,
+                                 uint32_t n_pixels, float exposure, float* image, cudaStream_t s);
 
 // bounce_graphs.cpp: step b of the wavefront loop b = 0 .. max_depth (single
 // job when jobs == nullptr, else batched) on `s`, replayed from a cached CUDA
