@@ -2,6 +2,7 @@
 // 38-118: built on first use, shared by every scene of the context) and the C
 // entry points that export them and query the device BSDF.
 #include <cmath>
+#include <algorithm>
 #include <cstring>
 
 #include "../host/openpbr_lower.h"
@@ -23,6 +24,21 @@ tpt_status upload_samples(tpt_context* ctx, const std::vector<float>& a, DevTabl
   if (st) return st;
   return cuda_check(ctx, cudaMemcpy(out->p, a.data(), a.size() * 4, cudaMemcpyHostToDevice), "cudaMemcpy(lut samples)");
 }
+
+// The lookup copy of a table of rows x cols cells, `layers` of them: per cell
+// itself, the next column, and the same two of the next row (clamped).
+std::vector<float> lookup_cells(const std::vector<float>& e, size_t layers, size_t rows, size_t cols) {
+  std::vector<float> out;
+  out.reserve(4 * e.size());
+  for (size_t l = 0; l < layers; ++l)
+    for (size_t r = 0; r < rows; ++r)
+      for (size_t c = 0; c < cols; ++c) {
+        const size_t r1 = std::min(r + 1, rows - 1), c1 = std::min(c + 1, cols - 1);
+        for (const size_t k : {r * cols + c, r * cols + c1, r1 * cols + c, r1 * cols + c1})
+          out.push_back(e[l * rows * cols + k]);
+      }
+  return out;
+}
 }  // namespace
 
 tpt_status ensure_ec_tables(tpt_context* ctx) {
@@ -36,10 +52,10 @@ tpt_status ensure_ec_tables(tpt_context* ctx) {
       (st = upload_samples(ctx, t.dec_cs, &dcs)))
     return st;
   float *cec = nullptr, *dec = nullptr;
-  if ((st = cuda_check(ctx, cudaMalloc(&cec, kCecLen * 4), "cudaMalloc(conductor table)"))) return st;
-  // the dielectric table with its E_avg behind it (the device's dispersive
-  // BTDF looks up E_avg at arbitrary etas)
-  if ((st = cuda_check(ctx, cudaMalloc(&dec, (kDecLen + kDecAvgLen) * 4), "cudaMalloc(dielectric table)"))) {
+  if ((st = cuda_check(ctx, cudaMalloc(&cec, kCecLen * 5 * 4), "cudaMalloc(conductor table)"))) return st;
+  // the tables with their lookup copies behind them, and the dielectric one's
+  // E_avg in between (the device's dispersive BTDF looks it up at arbitrary etas)
+  if ((st = cuda_check(ctx, cudaMalloc(&dec, (kDecLen * 5 + kDecAvgLen) * 4), "cudaMalloc(dielectric table)"))) {
     cudaFree(cec);
     return st;
   }
@@ -60,11 +76,18 @@ tpt_status ensure_ec_tables(tpt_context* ctx) {
   ctx->h_dec_e_avg.assign(kDecAvgLen, 0.0f);
   conductor_e_avg(ctx->h_cec_e.data(), ctx->h_cec_e_avg.data());
   dielectric_e_avg(ctx->h_dec_e.data(), ctx->h_dec_e_avg.data());
+  static_assert(kDecLookupBase == kDecLen + kDecAvgLen && kCecLookupBase == kCecLen, "lookup copies");
+  const std::vector<float> cec_cells = lookup_cells(ctx->h_cec_e, 1, 64, 64);
+  const std::vector<float> dec_cells = lookup_cells(ctx->h_dec_e, 32, 32, 32);
   e = cudaMemcpy(dec + kDecLen, ctx->h_dec_e_avg.data(), kDecAvgLen * 4, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess)
+    e = cudaMemcpy(cec + kCecLookupBase, cec_cells.data(), cec_cells.size() * 4, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess)
+    e = cudaMemcpy(dec + kDecLookupBase, dec_cells.data(), dec_cells.size() * 4, cudaMemcpyHostToDevice);
   if (e != cudaSuccess) {
     cudaFree(cec);
     cudaFree(dec);
-    return cuda_check(ctx, e, "dielectric E_avg upload");
+    return cuda_check(ctx, e, "table lookup upload");
   }
   ctx->d_cec_e = cec;
   ctx->d_dec_e = dec;
@@ -85,7 +108,7 @@ tpt_status ensure_da_table(tpt_context* ctx, float eta, const float** out) {
   tpt_status st;
   if ((st = upload_samples(ctx, t.da_dirs, &dirs)) || (st = upload_samples(ctx, t.da_phi_cs, &cs))) return st;
   float* tab = nullptr;
-  if ((st = cuda_check(ctx, cudaMalloc(&tab, (size_t)kDaLen * 4), "cudaMalloc(albedo table)"))) return st;
+  if ((st = cuda_check(ctx, cudaMalloc(&tab, (size_t)(kDaLen + kDaLookupLen) * 4), "cudaMalloc(albedo table)"))) return st;
   cudaError_t e = launch_lut_dielectric_albedo(eta, dirs.p, cs.p, tab, ctx->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
   if (e != cudaSuccess) {

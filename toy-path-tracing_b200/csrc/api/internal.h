@@ -251,6 +251,7 @@ tpt_status ensure_da_table(tpt_context* ctx, float eta, const float** out);
 
 // lut_kernels.cu: table construction (bit-exact with the reference's loops;
 // the sample tables come from lut_sample_tables).
+// out: the table, then its lookup copy (kDaLookupLen floats)
 cudaError_t launch_lut_dielectric_albedo(float eta, const float* dirs, const float* phi_cs, float* out,
                                          cudaStream_t s);
 cudaError_t launch_lut_conductor_e(const float* u, const float* cs, float* e, cudaStream_t s);

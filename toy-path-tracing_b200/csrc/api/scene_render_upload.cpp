@@ -109,6 +109,9 @@ tpt_status lower_openpbr_material(tpt_context* ctx, const tpt_openpbr_desc& d, D
   if (!st) st = ensure_da_table(ctx, openpbr_spec_table_eta(d), &spec_da);
   if (!st && d.coat_weight > 0.0f) st = ensure_da_table(ctx, openpbr_coat_table_eta(d), &coat_da);
   if (st) return st;
+  // lookups read the copy behind each table
+  if (spec_da) spec_da += kDaLen;
+  if (coat_da) coat_da += kDaLen;
   lower_openpbr(d, spec_da, coat_da, ctx->h_cec_e_avg.data(), ctx->h_dec_e_avg.data(), out);
   return TPT_OK;
 }

@@ -204,28 +204,35 @@ __device__ __forceinline__ DevLerpAxis axis_lerp(float value, int resolution) {
   return DevLerpAxis{(uint32_t)lower, (uint32_t)lower + 1u, position - (float)lower};
 }
 
-// DielectricGgxDirectionalAlbedoLut::lookup(w, roughness proxy, anisotropy 0)
+// DielectricGgxDirectionalAlbedoLut::lookup(w, roughness proxy, anisotropy 0).
+// Anisotropy 0 sits at position 7.5 of its 16 cells: indices 7 and 8, weights 1/2.
+//
+// The three tables are read through lookup copies whose entry holds the four
+// cells that two neighbouring indices on two axes give: 4, 2 and 1 loads of 16
+// bytes for the albedo, the dielectric and the conductor instead of 16, 8 and 4
+// words in as many sectors.  Where an axis is clamped its two indices are the
+// same and the second weight is zero, so that the copy's next cell adds exactly
+// the zero that the same cell would.
 static __device__ __noinline__ float da_lookup(const float* __restrict__ tab, float eta, bool smooth, DevLerpAxis r, V3 w) {
   if (w.z <= 0.0f) return 0.0f;
   if (smooth) return fresnel_dielectric(clampf(w.z, 0.0f, 1.0f), 1.0f, eta);
   const float sqrt_cos = sqrtf(clampf(w.z, 0.0f, 1.0f));
   const float phi = ((w.x == 0.0f && w.y == 0.0f) ? 0.0f : atan2f(fabsf(w.y), fabsf(w.x))) / kFracPi2;
   const DevLerpAxis c = axis_lerp(sqrt_cos, 64), p = axis_lerp(phi, 16);
-  const uint32_t ci[2] = {c.lo, c.hi}, pi[2] = {p.lo, p.hi}, ri[2] = {r.lo, r.hi};
+  const uint32_t ci[2] = {c.lo, c.hi}, pi[2] = {p.lo, p.hi};
   const float cw[2] = {1.0f - c.t, c.t}, pw[2] = {1.0f - p.t, p.t}, rw[2] = {1.0f - r.t, r.t};
   float value = 0.0f;
 #pragma unroll
   for (int x = 0; x < 2; ++x)
 #pragma unroll
-    for (int y = 0; y < 2; ++y)
-#pragma unroll
-      for (int z = 0; z < 2; ++z) {
-        // anisotropy 0 sits at position 7.5 of its 16 cells: indices 7 and 8, weights 1/2
-        const float* row = tab + ((size_t)(ci[x] * 16u + pi[y]) * 64u + ri[z]) * 16u;
-        const float wxyz = cw[x] * pw[y] * rw[z];
-        value += wxyz * 0.5f * __ldg(row + 7);
-        value += wxyz * 0.5f * __ldg(row + 8);
-      }
+    for (int y = 0; y < 2; ++y) {
+      const float4 cell = __ldg(reinterpret_cast<const float4*>(tab) + ((ci[x] * 16u + pi[y]) * 64u + r.lo));
+      const float w0 = cw[x] * pw[y] * rw[0], w1 = cw[x] * pw[y] * rw[1];
+      value += w0 * 0.5f * cell.x;
+      value += w0 * 0.5f * cell.y;
+      value += w1 * 0.5f * cell.z;
+      value += w1 * 0.5f * cell.w;
+    }
   return clampf(value, 0.0f, 1.0f);
 }
 
@@ -233,16 +240,19 @@ static __device__ __noinline__ float da_lookup(const float* __restrict__ tab, fl
 __device__ __forceinline__ float dec_lookup_e(const float* __restrict__ e, const DevMsFace& f, float cos_theta) {
   const float sqrt_cos = sqrtf(clampf(cos_theta, 0.0f, 1.0f));
   const DevLerpAxis c = axis_lerp(sqrt_cos, 32);
-  const uint32_t hi[2] = {f.eta_axis.lo, f.eta_axis.hi}, ri[2] = {f.r_axis.lo, f.r_axis.hi}, ci[2] = {c.lo, c.hi};
+  const uint32_t hi[2] = {f.eta_axis.lo, f.eta_axis.hi};
   const float hw[2] = {1.0f - f.eta_axis.t, f.eta_axis.t}, rw[2] = {1.0f - f.r_axis.t, f.r_axis.t},
               cw[2] = {1.0f - c.t, c.t};
   float value = 0.0f;
 #pragma unroll
-  for (int x = 0; x < 2; ++x)
-#pragma unroll
-    for (int y = 0; y < 2; ++y)
-#pragma unroll
-      for (int z = 0; z < 2; ++z) value += hw[x] * rw[y] * cw[z] * __ldg(e + (hi[x] * 32u + ri[y]) * 32u + ci[z]);
+  for (int x = 0; x < 2; ++x) {
+    const float4 cell = __ldg(reinterpret_cast<const float4*>(e + kDecLookupBase) +
+                              ((hi[x] * 32u + f.r_axis.lo) * 32u + c.lo));
+    value += hw[x] * rw[0] * cw[0] * cell.x;
+    value += hw[x] * rw[0] * cw[1] * cell.y;
+    value += hw[x] * rw[1] * cw[0] * cell.z;
+    value += hw[x] * rw[1] * cw[1] * cell.w;
+  }
   return clampf(value, 0.0f, 1.0f);
 }
 
@@ -250,13 +260,13 @@ __device__ __forceinline__ float dec_lookup_e(const float* __restrict__ e, const
 __device__ __forceinline__ float cec_lookup_e(const float* __restrict__ e, DevLerpAxis r, float cos_theta) {
   const float sqrt_cos = sqrtf(clampf(cos_theta, 0.0f, 1.0f));
   const DevLerpAxis c = axis_lerp(sqrt_cos, 64);
-  const uint32_t ci[2] = {c.lo, c.hi}, ri[2] = {r.lo, r.hi};
   const float cw[2] = {1.0f - c.t, c.t}, rw[2] = {1.0f - r.t, r.t};
+  const float4 cell = __ldg(reinterpret_cast<const float4*>(e + kCecLookupBase) + (r.lo * 64u + c.lo));
   float value = 0.0f;
-#pragma unroll
-  for (int x = 0; x < 2; ++x)
-#pragma unroll
-    for (int y = 0; y < 2; ++y) value += cw[x] * rw[y] * __ldg(e + ri[y] * 64u + ci[x]);
+  value += cw[0] * rw[0] * cell.x;
+  value += cw[0] * rw[1] * cell.z;
+  value += cw[1] * rw[0] * cell.y;
+  value += cw[1] * rw[1] * cell.w;
   return clampf(value, 0.0f, 1.0f);
 }
 

@@ -73,6 +73,9 @@ enum : uint32_t {
 // The dielectric energy-compensation table E (32 eta x 32 roughness x 32
 // sqrt cos); its E_avg (32 eta x 32 roughness) follows it in the same buffer.
 constexpr uint32_t kDecTableLen = 32u * 32u * 32u;
+// First float of the energy-compensation tables' lookup copies: behind E and E_avg
+// (dielectric) and behind E (conductor).
+constexpr uint32_t kDecLookupBase = kDecTableLen + 32u * 32u, kCecLookupBase = 64u * 64u;
 struct alignas(16) DevOpenPbr {
   float base_color[3], base;
   float specular, specular_color[3];
@@ -83,7 +86,7 @@ struct alignas(16) DevOpenPbr {
   float eon_r_pow01;  // r^0.1 of the EON uniform-lobe probability
   uint32_t flags;
   float spec_da_eta, coat_da_eta;  // etas of the albedo tables
-  const float* spec_da;            // directional albedo tables (64 x 16 x 64 x 16)
+  const float* spec_da;            // directional albedo lookups (64 x 16 x 64 x 4, da_lookup)
   const float* coat_da;
   DevLerpAxis spec_da_r, coat_da_r;  // roughness axis at the roughness proxies
   // metal (F82-tint Fresnel + conductor multiple scattering)

@@ -12,6 +12,9 @@
 namespace tpt {
 
 constexpr int kDaLen = 64 * 16 * 64 * 16;
+// Lookup copies the device keeps behind its tables: four cells per entry, the
+// ones an interpolation reads together (dec_lookup_e, cec_lookup_e, da_lookup).
+constexpr int kDaLookupLen = 64 * 16 * 64 * 4;
 constexpr int kCecLen = 64 * 64, kCecAvgLen = 64;
 constexpr int kDecLen = 32 * 32 * 32, kDecAvgLen = 32 * 32;
 

@@ -261,12 +261,23 @@ __global__ void __launch_bounds__(kLutBlock) lut_dec_kernel(const float* __restr
   }
   e[index] = val;
 }
+
+// The lookup copy of the albedo table: columns 7 and 8 (the two that anisotropy 0
+// lies between) of a roughness row and of the next.
+__global__ void __launch_bounds__(kLutBlock) lut_da_cells_kernel(const float* __restrict__ tab,
+                                                                 float4* __restrict__ out) {
+  const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= 64u * 16u * 64u) return;
+  const unsigned j = (i & 63u) == 63u ? i : i + 1u;
+  out[i] = make_float4(tab[16u * i + 7u], tab[16u * i + 8u], tab[16u * j + 7u], tab[16u * j + 8u]);
+}
 }  // namespace
 
 cudaError_t launch_lut_dielectric_albedo(float eta, const float* dirs, const float* phi_cs, float* out,
                                          cudaStream_t s) {
   const unsigned n = 64u * 16u * 64u * 16u;
   lut_da_kernel<<<(n + kLutBlock - 1) / kLutBlock, kLutBlock, 0, s>>>(eta, dirs, phi_cs, out);
+  lut_da_cells_kernel<<<(n / 16u + kLutBlock - 1) / kLutBlock, kLutBlock, 0, s>>>(out, (float4*)(out + n));
   return cudaGetLastError();
 }
 cudaError_t launch_lut_conductor_e(const float* u, const float* cs, float* e, cudaStream_t s) {
