@@ -84,6 +84,7 @@ tpt_status ensure_ec_tables(tpt_context* ctx) {
     e = cudaMemcpy(cec + kCecLookupBase, cec_cells.data(), cec_cells.size() * 4, cudaMemcpyHostToDevice);
   if (e == cudaSuccess)
     e = cudaMemcpy(dec + kDecLookupBase, dec_cells.data(), dec_cells.size() * 4, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);  // the copies' last bytes, for other streams
   if (e != cudaSuccess) {
     cudaFree(cec);
     cudaFree(dec);

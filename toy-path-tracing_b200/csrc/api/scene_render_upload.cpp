@@ -55,22 +55,37 @@ tpt_status put(tpt_scene* s, const std::vector<T>& v, const T** dst) {
   return TPT_OK;
 }
 
-// Device memory of one call.
+// Device memory of one call: the context's staging buffer up to 128 MiB (it stays
+// mapped between calls), memory of its own above.
 struct TempArrays {
   tpt_context* ctx;
-  std::vector<void*> ptrs;
+  char *p = nullptr, *base = nullptr;  // the next array's place, the block
+  bool own = false;
   explicit TempArrays(tpt_context* c) : ctx(c) {}
   ~TempArrays() {
-    for (void* p : ptrs) cudaFree(p);
+    if (own) cudaFree(base);
+  }
+  template <class T>
+  static size_t size_of(const std::vector<T>& v) {
+    return (v.size() * sizeof(T) + 255) & ~(size_t)255;
+  }
+  tpt_status take(size_t bytes) {
+    if (bytes <= (128u << 20)) {
+      tpt_status st = ensure_device_staging(ctx, std::max<size_t>(bytes, 16));
+      if (!st) p = (char*)ctx->d_stage;
+      return st;
+    }
+    tpt_status st = cuda_check(ctx, cudaMalloc((void**)&p, bytes), "cudaMalloc(upload)");
+    own = !st;
+    base = p;
+    return st;
   }
   template <class T>
   tpt_status put(const std::vector<T>& v, const T** dst) {
-    void* p = nullptr;
-    tpt_status st = cuda_check(ctx, cudaMalloc(&p, std::max<size_t>(v.size() * sizeof(T), 16)), "cudaMalloc(upload)");
-    if (st) return st;
-    ptrs.push_back(p);
     *dst = (const T*)p;
-    return cuda_check(ctx, cudaMemcpy(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice), "cudaMemcpy(upload)");
+    p += size_of(v);
+    return cuda_check(ctx, cudaMemcpy((void*)*dst, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice),
+                      "cudaMemcpy(upload)");
   }
 };
 
@@ -86,18 +101,21 @@ tpt_status put_shade_tris(tpt_scene* s, const std::vector<MeshSpan>& spans, cons
   void* out = nullptr;
   const uint64_t n = idx.size() / 3;
   tpt_status st = scene_alloc(s, n * sizeof(DevShadeTri), &out);
+  if (!st)
+    st = tmp.take(tmp.size_of(spans) + tmp.size_of(pos) + tmp.size_of(nrm) + tmp.size_of(uv) + tmp.size_of(idx));
   if (!st) st = tmp.put(spans, &d_spans);
   if (!st) st = tmp.put(pos, &d_pos);
   if (!st) st = tmp.put(nrm, &d_nrm);
   if (!st) st = tmp.put(uv, &d_uv);
   if (!st) st = tmp.put(idx, &d_idx);
   if (st) return st;
-  cudaStream_t stream = s->ctx->stream;
+  // on the copies' stream: a copy from pageable memory may return before its last
+  // bytes have reached the device
   st = cuda_check(s->ctx,
                   launch_bake_shade_tris(d_spans, (uint32_t)spans.size(), d_pos, d_nrm, d_uv, d_idx, n,
-                                         (DevShadeTri*)out, stream),
+                                         (DevShadeTri*)out, cudaStreamLegacy),
                   "shading record launch");
-  if (!st) st = cuda_check(s->ctx, cudaStreamSynchronize(stream), "shading records");
+  if (!st) st = cuda_check(s->ctx, cudaStreamSynchronize(cudaStreamLegacy), "shading records");
   *dst = (const DevShadeTri*)out;
   return st;
 }
