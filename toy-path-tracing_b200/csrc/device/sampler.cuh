@@ -152,8 +152,13 @@ __device__ __forceinline__ void sample_index32(uint32_t morton, uint32_t log2_sp
   }
 }
 
-// IndexSampler (zsobol.rs:206-285) + PathSampler (path_sampler.rs:146-250)
-struct PathSamplerDev {
+// IndexSampler (zsobol.rs:206-285) + PathSampler (path_sampler.rs:146-250).
+// ANY: the pixel and sample may lie outside the image, whose Morton index can be
+// longer than the image's digits; a digit's permutation depends on every bit above
+// it, so such an index takes the 64-bit loop.  Render paths lie inside by
+// construction and leave the check out.
+template <bool ANY>
+struct PathSampler {
   uint64_t morton;  // (encode_morton_2(px, py) << log2_spp) | sample
   uint32_t log2_spp;
   uint32_t n_base4_digits;
@@ -183,7 +188,10 @@ struct PathSamplerDev {
     return out;
   }
 
-  __device__ __forceinline__ bool narrow() const { return 2u * n_base4_digits - (log2_spp & 1u) <= 32u; }
+  __device__ __forceinline__ bool narrow() const {
+    const uint32_t bits = 2u * n_base4_digits - (log2_spp & 1u);
+    return bits <= 32u && (!ANY || (morton >> bits) == 0);
+  }
 
   // sample_index of N dimensions, its words folded by xor
   template <int N>
@@ -209,7 +217,7 @@ struct PathSamplerDev {
   }
   // Out of line and by value: a draw is some 400 instructions, and a shading
   // vertex makes several; the kernels keep one copy of each form.
-  static __device__ __noinline__ float draw_1(PathSamplerDev s, uint32_t dim) {
+  static __device__ __noinline__ float draw_1(PathSampler s, uint32_t dim) {
     const uint32_t d[1] = {dim};
     uint32_t i[1];
     s.folded_indices<1>(d, i);
@@ -217,7 +225,7 @@ struct PathSamplerDev {
     s.point<false>(dim, i[0], a, b);
     return a;
   }
-  static __device__ __noinline__ float2 draw_2(PathSamplerDev s, uint32_t dim) {
+  static __device__ __noinline__ float2 draw_2(PathSampler s, uint32_t dim) {
     const uint32_t d[1] = {dim};
     uint32_t i[1];
     s.folded_indices<1>(d, i);
@@ -227,7 +235,7 @@ struct PathSamplerDev {
   }
   // a 2D and a 1D draw (z) of one vertex together: the digit's share of the work
   // once, and two independent chains for the scheduler
-  static __device__ __noinline__ float3 draw_21(PathSamplerDev s, uint32_t dim2, uint32_t dim1) {
+  static __device__ __noinline__ float3 draw_21(PathSampler s, uint32_t dim2, uint32_t dim1) {
     const uint32_t d[2] = {dim2, dim1};
     uint32_t i[2];
     s.folded_indices<2>(d, i);
@@ -238,7 +246,7 @@ struct PathSamplerDev {
     return r;
   }
   // 1D draws of four consecutive dimensions
-  static __device__ __noinline__ float4 draw_1111(PathSamplerDev s, uint32_t dim) {
+  static __device__ __noinline__ float4 draw_1111(PathSampler s, uint32_t dim) {
     const uint32_t d[4] = {dim, dim + 1u, dim + 2u, dim + 3u};
     uint32_t i[4];
     s.folded_indices<4>(d, i);
@@ -277,6 +285,7 @@ struct PathSamplerDev {
     return pcg_hash((uint32_t)bits ^ (uint32_t)(bits >> 32));
   }
 };
+using PathSamplerDev = PathSampler<false>;
 
 // Dimension layout (path_sampler.rs:153-169): camera at 0, vertex `depth` at
 // 2 + 16 * depth + offset.

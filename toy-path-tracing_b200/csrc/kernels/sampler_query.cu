@@ -8,8 +8,8 @@
 // then camera_sample (dimension 0), initial_aux_rng_seed (dimension
 // 0x80000000) and path_vertex_randoms(depth) (path_sampler.rs:97-118: the 11
 // values at 2 + 16 depth + {0..13} and the aux seed at + 14) -- the same
-// PathSamplerDev calls, with the same dimension numbers, that the render
-// kernels make.
+// sampler calls, with the same dimension numbers, that the render kernels make.
+// Queries may name pixels and samples outside the image: PathSampler<true>.
 #include <algorithm>
 
 #include "../api/internal.h"
@@ -26,7 +26,7 @@ __global__ void sampler_values_kernel(uint32_t log2_spp, uint32_t n_digits, uint
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const uint4 q = queries[i];  // px, py, sample, depth
-  PathSamplerDev ps;
+  PathSampler<true> ps;
   ps.init(q.x, q.y, q.z, log2_spp, n_digits);
   float v[16];
   ps.sample_2d(kDimCamera, v[0], v[1]);
