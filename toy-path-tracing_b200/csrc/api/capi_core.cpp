@@ -66,18 +66,38 @@ unsigned long long* next_counter(tpt_context* ctx) {
   return ctx->d_counters + k;
 }
 
-tpt_status ensure_device_staging(tpt_context* ctx, size_t bytes) {
-  if (ctx->d_stage_bytes >= bytes) return TPT_OK;
-  if (ctx->d_stage) {
-    cudaStreamSynchronize(ctx->stream);
-    cudaFree(ctx->d_stage);
+tpt_status CallBlock::take(size_t n) {
+  n = std::max<size_t>(n, 16);
+  if (n <= kKeptBytes) {
+    std::lock_guard<std::mutex> g(ctx->block_mu);
+    p = (char*)ctx->block;
+    bytes = ctx->block_bytes;
+    ctx->block = nullptr;
+    ctx->block_bytes = 0;
   }
-  ctx->d_stage = nullptr;
-  ctx->d_stage_bytes = 0;
-  tpt_status st = cuda_check(ctx, cudaMalloc(&ctx->d_stage, bytes), "cudaMalloc(staging)");
-  if (st) return st;
-  ctx->d_stage_bytes = bytes;
-  return TPT_OK;
+  if (bytes >= n) return TPT_OK;
+  if (p) cudaFree(p);
+  p = nullptr;
+  bytes = 0;
+  tpt_status st = cuda_check(ctx, cudaMalloc((void**)&p, n), "cudaMalloc(call memory)");
+  if (st) p = nullptr;
+  else bytes = n;
+  return st;
+}
+
+CallBlock::~CallBlock() {
+  if (!p) return;
+  cudaStreamSynchronize(stream);
+  if (bytes <= kKeptBytes) {
+    std::lock_guard<std::mutex> g(ctx->block_mu);
+    if (bytes > ctx->block_bytes) {
+      void* smaller = ctx->block;
+      ctx->block = p;
+      ctx->block_bytes = bytes;
+      p = (char*)smaller;
+    }
+  }
+  if (p) cudaFree(p);
 }
 
 }  // namespace tpt
@@ -158,6 +178,20 @@ tpt_status ensure_host_staging(tpt_context* ctx, size_t bytes) {
   tpt_status st = cuda_check(ctx, cudaMallocHost(&ctx->h_stage, bytes), "cudaMallocHost(staging)");
   if (st) return st;
   ctx->h_stage_bytes = bytes;
+  return TPT_OK;
+}
+
+tpt_status ensure_device_staging(tpt_context* ctx, size_t bytes) {
+  if (ctx->d_stage_bytes >= bytes) return TPT_OK;
+  if (ctx->d_stage) {
+    cudaStreamSynchronize(ctx->stream);
+    cudaFree(ctx->d_stage);
+  }
+  ctx->d_stage = nullptr;
+  ctx->d_stage_bytes = 0;
+  tpt_status st = cuda_check(ctx, cudaMalloc(&ctx->d_stage, bytes), "cudaMalloc(staging)");
+  if (st) return st;
+  ctx->d_stage_bytes = bytes;
   return TPT_OK;
 }
 
@@ -383,6 +417,7 @@ tpt_status tpt_context_destroy(tpt_context* ctx) {
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
   if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
   if (ctx->d_stage) cudaFree(ctx->d_stage);
+  if (ctx->block) cudaFree(ctx->block);
   if (ctx->d_err) cudaFree(ctx->d_err);
   destroy_bounce_graphs(ctx);
   if (ctx->d_counters) cudaFree(ctx->d_counters);

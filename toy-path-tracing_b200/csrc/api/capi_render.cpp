@@ -315,28 +315,26 @@ tpt_status render_launch_params(tpt_context* ctx, const tpt_render_job* job, Ren
   return make_launch(ctx, job, out);
 }
 
-// Device memory of a host-image render's images, on the context's stream.  Up to
-// kKeptImageBytes (a 4K image and more) it is the context's staging buffer, kept
-// between calls: memory from the default pool is unmapped again at the call's
-// final synchronisation, which cost a 97x61 preview more (0.5-1.5 ms) than its
-// rendering (0.7 ms).  Larger images are allocated and freed in the call.
+// Device memory of a host-image render's images, on the context's stream: a block
+// lent by the context up to CallBlock::kKeptBytes (memory from the default pool is
+// unmapped again at the call's final synchronisation, which cost a 97x61 preview
+// more, 0.5-1.5 ms, than its rendering, 0.7 ms), above that memory of the call's own.
 struct ImageMemory {
-  static constexpr size_t kKeptImageBytes = 128u << 20;
-  tpt_context* ctx;
+  CallBlock block;
   char* p = nullptr;
   bool own = false;
-  explicit ImageMemory(tpt_context* c) : ctx(c) {}
+  explicit ImageMemory(tpt_context* c) : block(c, c->stream) {}
   tpt_status take(size_t bytes) {
-    if (bytes <= kKeptImageBytes) {
-      tpt_status st = ensure_device_staging(ctx, std::max<size_t>(bytes, 16));
-      if (!st) p = (char*)ctx->d_stage;
+    if (bytes <= CallBlock::kKeptBytes) {
+      tpt_status st = block.take(bytes);
+      p = block.p;
       return st;
     }
     own = true;
-    return cuda_check(ctx, cudaMallocAsync((void**)&p, bytes, ctx->stream), "cudaMallocAsync(image)");
+    return cuda_check(block.ctx, cudaMallocAsync((void**)&p, bytes, block.stream), "cudaMallocAsync(image)");
   }
-  void give_back() {
-    if (own && p) cudaFreeAsync(p, ctx->stream);
+  void give_back() {  // before the call's last synchronisation, which unmaps memory of its own
+    if (own && p) cudaFreeAsync(p, block.stream);
     p = nullptr;
   }
 };

@@ -4,6 +4,7 @@
 
 #include <cstdint>
 #include <map>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -35,8 +36,12 @@ struct tpt_context {
   // pinned staging for the host-pointer entry points
   void* h_stage = nullptr;
   size_t h_stage_bytes = 0;
-  void* d_stage = nullptr;
+  void* d_stage = nullptr;  // tpt_traverse's rays and results on the device
   size_t d_stage_bytes = 0;
+  // one device block of at most tpt::CallBlock::kKeptBytes that no call uses at the moment
+  std::mutex block_mu;
+  void* block = nullptr;
+  size_t block_bytes = 0;
   cudaStream_t pipe[2] = {nullptr, nullptr};  // copy/compute pipeline of tpt_traverse
   cudaEvent_t ev_slot[2] = {nullptr, nullptr};
   cudaEvent_t ev_start = nullptr;
@@ -130,9 +135,23 @@ tpt_status cuda_check(tpt_context* ctx, cudaError_t e, const char* what);
 tpt_status check_device_errors(tpt_context* ctx, cudaStream_t stream);
 // Records that entry point `name` queued device work whose checks are read later.
 void note_device_call(tpt_context* ctx, const char* name);
-// Grows the context's device staging buffer (ctx->d_stage), which host-buffer
-// calls use and have finished with when they return.
-tpt_status ensure_device_staging(tpt_context* ctx, size_t bytes);
+// Device memory of one call, whose work on it runs on `stream` (or is waited for
+// there).  Up to kKeptBytes it is lent from the context, which keeps the block
+// for the next call: mapping and unmapping memory costs a small call more than
+// its work.  A block belongs to one call at a time, so calls of several threads
+// do not share it (the larger of two given back is kept), and the destructor
+// waits for `stream` before giving it back, on error exits too.
+struct CallBlock {
+  static constexpr size_t kKeptBytes = 128u << 20;  // a 4K image and more
+  tpt_context* ctx;
+  cudaStream_t stream;
+  char* p = nullptr;
+  size_t bytes = 0;
+  CallBlock(tpt_context* c, cudaStream_t s) : ctx(c), stream(s) {}
+  CallBlock(const CallBlock&) = delete;
+  ~CallBlock();
+  tpt_status take(size_t n);
+};
 // cudaSetDevice(ctx->device) with its status checked.
 tpt_status set_device(tpt_context* ctx);
 

@@ -55,36 +55,25 @@ tpt_status put(tpt_scene* s, const std::vector<T>& v, const T** dst) {
   return TPT_OK;
 }
 
-// Device memory of one call: the context's staging buffer up to 128 MiB (it stays
-// mapped between calls), memory of its own above.
+// Arrays that one call needs on the device, one after the other in a block.
 struct TempArrays {
-  tpt_context* ctx;
-  char *p = nullptr, *base = nullptr;  // the next array's place, the block
-  bool own = false;
-  explicit TempArrays(tpt_context* c) : ctx(c) {}
-  ~TempArrays() {
-    if (own) cudaFree(base);
-  }
+  CallBlock block;
+  char* p = nullptr;  // the next array's place
+  explicit TempArrays(tpt_context* c) : block(c, cudaStreamLegacy) {}
   template <class T>
   static size_t size_of(const std::vector<T>& v) {
     return (v.size() * sizeof(T) + 255) & ~(size_t)255;
   }
   tpt_status take(size_t bytes) {
-    if (bytes <= (128u << 20)) {
-      tpt_status st = ensure_device_staging(ctx, std::max<size_t>(bytes, 16));
-      if (!st) p = (char*)ctx->d_stage;
-      return st;
-    }
-    tpt_status st = cuda_check(ctx, cudaMalloc((void**)&p, bytes), "cudaMalloc(upload)");
-    own = !st;
-    base = p;
+    tpt_status st = block.take(bytes);
+    p = block.p;
     return st;
   }
   template <class T>
   tpt_status put(const std::vector<T>& v, const T** dst) {
     *dst = (const T*)p;
     p += size_of(v);
-    return cuda_check(ctx, cudaMemcpy((void*)*dst, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice),
+    return cuda_check(block.ctx, cudaMemcpy((void*)*dst, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice),
                       "cudaMemcpy(upload)");
   }
 };
