@@ -226,7 +226,7 @@ tpt_status call(const std::string& what) {
     tpt_scene_release(s);
     return st;
   }
-  const int side = what == "render_large" ? 2000 : 64, jobs = what == "render_batch" ? 3 : 1;
+  const int side = what == "render_large" ? 2000 : what == "render_own_memory" ? 3400 : 64, jobs = what == "render_batch" ? 3 : 1;
   tpt_render_job j{};
   j.scene = scene;
   j.camera.look_at[2] = -1.0f;

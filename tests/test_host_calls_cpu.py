@@ -3,6 +3,7 @@ C++ objects linked with a stand-in of the CUDA runtime (host_calls_fake.cpp).
 
 * A host call begun while another of the same context is in flight (as a second
   thread does) leaves the other's memory alone.
+* A call that fails half-way returns its error with nothing of its work in flight.
 """
 import os
 import subprocess
@@ -40,3 +41,11 @@ def run(program, *args):
 ])
 def test_calls_in_flight_keep_their_memory(program, outer, inner):
     run(program, "share", outer, inner)
+
+
+# three or more launches: a query of 300,001 rays in chunks, one traversal per bounce
+# and the image of a render, three jobs of a batch
+@pytest.mark.parametrize("call", ["traverse_pinned", "traverse_pageable", "render", "render_own_memory", "render_batch"])
+@pytest.mark.parametrize("launch", [1, 2, 3])
+def test_failed_calls_leave_nothing_in_flight(program, call, launch):
+    run(program, "fail", call, str(launch))

@@ -247,6 +247,23 @@ tpt_status ensure_copy_pipeline(tpt_context* ctx, size_t n_chunks) {
 
 bool is_pinned(const void* p);
 
+// Waits for a query's streams when the call leaves on an error: copies and kernels
+// that are queued still work on the caller's arrays, the context's staging buffers
+// (which the next call refills) and the scene.
+struct QueryExit {
+  tpt_context* ctx;
+  bool queued = true;  // work that has not been waited for
+  ~QueryExit() {
+    if (!queued) return;
+    for (cudaStream_t s : {ctx->copy_in, ctx->pipe[0], ctx->pipe[1], ctx->copy_out, ctx->stream})
+      if (s) cudaStreamSynchronize(s);
+  }
+  tpt_status done(tpt_status st) {  // what the last wait returned
+    queued = st != TPT_OK;
+    return st;
+  }
+};
+
 }  // namespace
 
 cudaMemPool_t tpt::build_pool(tpt_context* ctx) {
@@ -774,6 +791,7 @@ tpt_status tpt_traverse(tpt_context* ctx, const tpt_scene* scene, const float* r
   tpt_status st = set_device(ctx);
   if (!st) st = ensure_pipeline(ctx);
   if (st) return st;
+  QueryExit exit{ctx};
   // Device buffers for the whole batch: rays (7 planes) then outputs.
   const int n_out = 2 + (instance ? 1 : 0) + (bary ? 3 : 0);
   const size_t dev_bytes = (7 + (size_t)n_out) * n * 4;
@@ -833,7 +851,7 @@ tpt_status tpt_traverse(tpt_context* ctx, const tpt_scene* scene, const float* r
     cudaEventRecord(ctx->ev_slot[0], ctx->copy_out);
     cudaStreamWaitEvent(ctx->stream, ctx->ev_slot[0], 0);
     if ((st = cuda_check(ctx, cudaGetLastError(), "traverse pipeline"))) return st;
-    return check_device_errors(ctx, ctx->stream);
+    return exit.done(check_device_errors(ctx, ctx->stream));
   }
   // Pageable buffers: pinned staging slots, pipelined on two streams: chunk c is
   // staged and queued while chunk c - 1 is on the device, and chunk c - 1's
@@ -887,7 +905,7 @@ tpt_status tpt_traverse(tpt_context* ctx, const tpt_scene* scene, const float* r
     cudaStreamWaitEvent(ctx->stream, ctx->ev_slot[k], 0);
   }
   if ((st = cuda_check(ctx, cudaGetLastError(), "traverse pipeline"))) return st;
-  return check_device_errors(ctx, ctx->stream);
+  return exit.done(check_device_errors(ctx, ctx->stream));
 }
 
 }  // extern "C"

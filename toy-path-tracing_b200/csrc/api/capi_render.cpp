@@ -338,6 +338,14 @@ struct ImageMemory {
     p = nullptr;
   }
 };
+
+// The end of a host-image render, after an error too: copies into the caller's
+// images may be queued.
+tpt_status finish_images(tpt_context* ctx, tpt_status st) {
+  if (!st) return check_device_errors(ctx, ctx->stream);
+  cudaStreamSynchronize(ctx->stream);
+  return st;
+}
 }  // namespace tpt
 
 extern "C" {
@@ -475,7 +483,7 @@ tpt_status tpt_render(tpt_context* ctx, const tpt_render_job* jobs, int n_jobs, 
                                            cudaMemcpyDeviceToHost, ctx->stream),
                       "D2H image");
     mem.give_back();
-    if (!st) st = check_device_errors(ctx, ctx->stream);
+    st = finish_images(ctx, st);
     return st;
   }
   for (int j = 0; j < n_jobs; ++j) {
@@ -491,7 +499,7 @@ tpt_status tpt_render(tpt_context* ctx, const tpt_render_job* jobs, int n_jobs, 
       st = cuda_check(ctx, cudaMemcpyAsync(out_rgb[j], mem.p, img_bytes, cudaMemcpyDeviceToHost, ctx->stream),
                       "D2H image");
     mem.give_back();
-    if (!st) st = check_device_errors(ctx, ctx->stream);
+    st = finish_images(ctx, st);
     if (st) return st;
   }
   return TPT_OK;
