@@ -7,6 +7,7 @@
 //   host_calls_fake share <outer> <inner>   one call begun while another is in
 //       flight on the same context, as by a second thread
 //   host_calls_fake fail <call> <k>         the k-th launch of a call fails
+//   host_calls_fake wait <call> 1           a call alone
 #include <cuda_runtime.h>
 
 #include <cstdio>
@@ -98,21 +99,24 @@ cudaError_t cudaMallocAsync(void** p, size_t n, cudaStream_t) { return get(p, n)
 cudaError_t cudaFree(void* p) { return drop(p); }
 cudaError_t cudaFreeHost(void* p) { return drop(p); }
 cudaError_t cudaFreeAsync(void* p, cudaStream_t) { return drop(p); }
+cudaError_t cudaStreamSynchronize(cudaStream_t s) { join(done, streams[s]); return cudaSuccess; }
 cudaError_t cudaMemset(void* p, int v, size_t n) { touch(p); std::memset(p, v, n); return cudaSuccess; }
 cudaError_t cudaMemsetAsync(void* p, int v, size_t n, cudaStream_t s) { issue(s); return cudaMemset(p, v, n); }
-cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) {
+cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t st) {
+  issue(st);
   touch(d);
   std::memcpy(d, s, n);
   return cudaSuccess;
 }
-cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind k, cudaStream_t st) {
-  issue(st);
-  return cudaMemcpy(d, s, n, k);
+// a copy from pageable memory returns when it has read the memory: its last bytes
+// may reach the device later, in the order of the legacy stream
+cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind k) {
+  cudaMemcpyAsync(d, s, n, k, cudaStreamLegacy);
+  return k == cudaMemcpyHostToDevice ? cudaSuccess : cudaStreamSynchronize(cudaStreamLegacy);
 }
 cudaError_t cudaMemcpy2DAsync(void* d, size_t dp, const void* s, size_t sp, size_t w, size_t h, cudaMemcpyKind k,
                               cudaStream_t st) {
-  issue(st);
-  for (size_t r = 0; r < h; ++r) cudaMemcpy((char*)d + r * dp, (const char*)s + r * sp, w, k);
+  for (size_t r = 0; r < h; ++r) cudaMemcpyAsync((char*)d + r * dp, (const char*)s + r * sp, w, k, st);
   return cudaSuccess;
 }
 cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void*) {
@@ -125,7 +129,6 @@ cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) {
   return cudaSuccess;
 }
 cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
-cudaError_t cudaStreamSynchronize(cudaStream_t s) { join(done, streams[s]); return cudaSuccess; }
 cudaError_t cudaDeviceSynchronize() {
   for (auto& [s, c] : streams) join(done, c);
   return cudaSuccess;
@@ -259,6 +262,8 @@ int main(int argc, char** argv) {
     if (call(what) || inner) return bad("a call failed");
     if (call(what) || call(arg)) return bad("a later call failed");
     if (!failure.empty()) return bad(failure.c_str());
+  } else if (mode == "wait") {
+    if (call(what)) return bad("a call failed");
   } else {
     fail_launch = std::atoi(argv[3]);
     const bool failed = call(what) != TPT_OK;

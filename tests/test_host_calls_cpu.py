@@ -4,6 +4,7 @@ C++ objects linked with a stand-in of the CUDA runtime (host_calls_fake.cpp).
 * A host call begun while another of the same context is in flight (as a second
   thread does) leaves the other's memory alone.
 * A call that fails half-way returns its error with nothing of its work in flight.
+* A call that succeeds does so too: a scene can be used on any stream at once.
 """
 import os
 import subprocess
@@ -49,3 +50,9 @@ def test_calls_in_flight_keep_their_memory(program, outer, inner):
 @pytest.mark.parametrize("launch", [1, 2, 3])
 def test_failed_calls_leave_nothing_in_flight(program, call, launch):
     run(program, "fail", call, str(launch))
+
+
+@pytest.mark.parametrize("call", ["upload", "upload_large", "traverse_pinned", "traverse_pageable", "render",
+                                  "render_own_memory", "render_batch"])
+def test_calls_leave_nothing_in_flight(program, call):
+    run(program, "wait", call, "1")

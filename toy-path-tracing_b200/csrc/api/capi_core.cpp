@@ -699,6 +699,9 @@ tpt_status tpt_scene_upload(tpt_context* ctx, const tpt_scene_desc* desc, tpt_sc
   s->geo.tlas_root_word = tlas_root;
   s->geo.num_instances = desc->num_instances;
   st = upload_render_data(s, desc);
+  // the copies are from pageable memory: the last bytes of each may reach the device
+  // after it has returned, and the scene may be used on any stream from here on
+  if (!st) st = cuda_check(ctx, cudaStreamSynchronize(cudaStreamLegacy), "scene upload");
   if (st) {
     tpt_scene_release(s);
     return st;

@@ -100,13 +100,11 @@ tpt_status put_shade_tris(tpt_scene* s, const std::vector<MeshSpan>& spans, cons
   if (st) return st;
   // on the copies' stream: a copy from pageable memory may return before its last
   // bytes have reached the device
-  st = cuda_check(s->ctx,
-                  launch_bake_shade_tris(d_spans, (uint32_t)spans.size(), d_pos, d_nrm, d_uv, d_idx, n,
-                                         (DevShadeTri*)out, cudaStreamLegacy),
-                  "shading record launch");
-  if (!st) st = cuda_check(s->ctx, cudaStreamSynchronize(cudaStreamLegacy), "shading records");
   *dst = (const DevShadeTri*)out;
-  return st;
+  return cuda_check(s->ctx,
+                    launch_bake_shade_tris(d_spans, (uint32_t)spans.size(), d_pos, d_nrm, d_uv, d_idx, n,
+                                           (DevShadeTri*)out, cudaStreamLegacy),
+                    "shading record launch");
 }
 }  // namespace
 
