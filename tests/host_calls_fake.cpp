@@ -8,6 +8,8 @@
 //       flight on the same context, as by a second thread
 //   host_calls_fake fail <call> <k>         the k-th launch of a call fails
 //   host_calls_fake wait <call> 1           a call alone
+//   host_calls_fake records <t> <bytes>     <bytes> a triangle are what a scene of <t>
+//       triangles with a material holds over one without
 #include <cuda_runtime.h>
 
 #include <cstdio>
@@ -187,7 +189,7 @@ namespace {
 tpt_context* ctx;
 tpt_scene* scene;
 
-tpt_status upload(uint32_t triangles, tpt_scene** out) {
+tpt_status upload(uint32_t triangles, tpt_scene** out, uint32_t materials = 1) {
   std::vector<float> p(9 * (size_t)triangles);
   std::vector<uint32_t> idx(3 * (size_t)triangles);
   for (uint32_t t = 0; t < triangles; ++t) {
@@ -211,7 +213,7 @@ tpt_status upload(uint32_t triangles, tpt_scene** out) {
   d.instances = &inst;
   d.num_instances = 1;
   d.materials = &mat;
-  d.num_materials = 1;
+  d.num_materials = materials;
   return tpt_scene_upload(ctx, &d, out);
 }
 
@@ -264,6 +266,13 @@ int main(int argc, char** argv) {
     if (!failure.empty()) return bad(failure.c_str());
   } else if (mode == "wait") {
     if (call(what)) return bad("a call failed");
+  } else if (mode == "records") {
+    tpt_scene *a = nullptr, *b = nullptr;
+    uint64_t with = 0, without = 0;
+    const uint64_t t = std::atoi(argv[2]), bytes = std::atoi(argv[3]);
+    if (upload(t, &a) || upload(t, &b, 0) || tpt_scene_device_bytes(a, &with) || tpt_scene_device_bytes(b, &without))
+      return bad("a call failed");
+    if (with < without + bytes * t) return bad("a scene for queries alone holds shading records");
   } else {
     fail_launch = std::atoi(argv[3]);
     const bool failed = call(what) != TPT_OK;

@@ -5,6 +5,7 @@ C++ objects linked with a stand-in of the CUDA runtime (host_calls_fake.cpp).
   thread does) leaves the other's memory alone.
 * A call that fails half-way returns its error with nothing of its work in flight.
 * A call that succeeds does so too: a scene can be used on any stream at once.
+* A scene without materials, which nothing can shade, holds no shading records.
 """
 import os
 import subprocess
@@ -56,3 +57,8 @@ def test_failed_calls_leave_nothing_in_flight(program, call, launch):
                                   "render_own_memory", "render_batch"])
 def test_calls_leave_nothing_in_flight(program, call):
     run(program, "wait", call, "1")
+
+
+@pytest.mark.parametrize("triangles", [100, 5000])
+def test_scenes_for_queries_hold_no_shading_records(program, triangles):
+    run(program, "records", str(triangles), "96")

@@ -78,8 +78,8 @@ struct TempArrays {
   }
 };
 
-// The shading records: the vertex arrays go to the device as they are (a fifth
-// of the records' size for a closed mesh) and are gathered there.
+// The shading records: the vertex arrays go to the device as they are (28 bytes
+// a triangle of a closed mesh, against the record's 96) and are gathered there.
 tpt_status put_shade_tris(tpt_scene* s, const std::vector<MeshSpan>& spans, const std::vector<float>& pos,
                           const std::vector<float>& nrm, const std::vector<float>& uv,
                           const std::vector<uint32_t>& idx, const DevShadeTri** dst) {
@@ -333,7 +333,8 @@ tpt_status upload_render_data(tpt_scene* s, const tpt_scene_desc* desc) {
   DevRenderData& R = s->render;
   tpt_status st = TPT_OK;
   if (!st) st = put(s, sinst, &R.inst);
-  if (!st) st = put_shade_tris(s, spans, pos, nrm, uv, idx, &R.tris);
+  // a scene without materials serves ray queries alone, which never read them
+  if (!st && desc->num_materials) st = put_shade_tris(s, spans, pos, nrm, uv, idx, &R.tris);
   if (!st) st = put(s, dmats, &R.mats);
   if (!st) st = put(s, lnodes, &R.ltree);
   if (!st) st = put(s, emap, &R.emitter_leaf);
