@@ -67,6 +67,13 @@ tpt_status tpt_context_destroy(tpt_context* ctx);
  * it after a `*_device` call's work (or a captured graph's replay) has been
  * ordered on `stream`; it cannot be called inside a stream capture. */
 tpt_status tpt_context_check(tpt_context* ctx, void* stream);
+/* Gives back the memory that host-buffer calls leave with the context for the
+ * next such call: the device buffer of tpt_traverse (as large as its largest
+ * batch) with its page-locked staging, and one device block of at most 128 MiB
+ * for host images and scene uploads.  Work that needs it allocates it again.
+ * Not to be called while a tpt_traverse of the same context runs.  (The arenas
+ * of renders stay; tpt_context_destroy frees everything.) */
+tpt_status tpt_context_trim(tpt_context* ctx);
 /* Message of the last failed call on `ctx` (or of the last failed context-less
  * call when ctx is NULL).  Valid until the next call on the same context. */
 const char* tpt_last_error(const tpt_context* ctx);

@@ -8,6 +8,8 @@
 //       flight on the same context, as by a second thread
 //   host_calls_fake fail <call> <k>         the k-th launch of a call fails
 //   host_calls_fake wait <call> 1           a call alone
+//   host_calls_fake trim <call> <mib>       what a call keeps is at most <mib> MiB and
+//       goes back with tpt_context_trim
 //   host_calls_fake records <t> <bytes>     <bytes> a triangle are what a scene of <t>
 //       triangles with a material holds over one without
 #include <cuda_runtime.h>
@@ -51,6 +53,11 @@ char* block_of(const void* p) {
   if (it == blocks.begin()) return nullptr;
   --it;
   return (char*)p < it->first + it->second ? it->first : nullptr;
+}
+size_t live_bytes() {
+  size_t n = 0;
+  for (auto& [p, bytes] : blocks) n += bytes;
+  return n;
 }
 void touch(const void* p) {
   if (char* b = block_of(p); b && in_use.count(b)) failure = "memory of a call in flight is written by another";
@@ -266,6 +273,15 @@ int main(int argc, char** argv) {
     if (!failure.empty()) return bad(failure.c_str());
   } else if (mode == "wait") {
     if (call(what)) return bad("a call failed");
+  } else if (mode == "trim") {
+    const size_t most = (size_t)std::atoi(argv[3]) << 20;
+    if (call(what) || tpt_context_trim(ctx)) return bad("a call failed");
+    const size_t before = live_bytes();  // arenas of renders stay
+    if (call(what)) return bad("a call failed");
+    if (live_bytes() == before || live_bytes() > before + most) return bad("memory kept by the call");
+    if (tpt_context_trim(ctx)) return bad("a call failed");
+    if (live_bytes() != before) return bad("memory not given back");
+    if (call(what)) return bad("a call after it failed");
   } else if (mode == "records") {
     tpt_scene *a = nullptr, *b = nullptr;
     uint64_t with = 0, without = 0;

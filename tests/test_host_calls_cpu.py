@@ -5,6 +5,7 @@ C++ objects linked with a stand-in of the CUDA runtime (host_calls_fake.cpp).
   thread does) leaves the other's memory alone.
 * A call that fails half-way returns its error with nothing of its work in flight.
 * A call that succeeds does so too: a scene can be used on any stream at once.
+* What calls keep for the next one is bounded and goes back with tpt_context_trim.
 * A scene without materials, which nothing can shade, holds no shading records.
 """
 import os
@@ -62,3 +63,10 @@ def test_calls_leave_nothing_in_flight(program, call):
 @pytest.mark.parametrize("triangles", [100, 5000])
 def test_scenes_for_queries_hold_no_shading_records(program, triangles):
     run(program, "records", str(triangles), "96")
+
+
+# a query of 300,001 rays: 7 + 2 planes on the device, 9 planes of two chunks in staging
+@pytest.mark.parametrize("call,mib", [("upload", 128), ("upload_large", 128), ("render", 128), ("render_large", 128),
+                                      ("render_batch", 128), ("traverse_pinned", 11), ("traverse_pageable", 16)])
+def test_kept_memory_is_bounded_and_given_back(program, call, mib):
+    run(program, "trim", call, str(mib))

@@ -467,6 +467,26 @@ tpt_status tpt_context_check(tpt_context* ctx, void* stream) {
   return check_device_errors(ctx, stream ? (cudaStream_t)stream : ctx->stream);
 }
 
+tpt_status tpt_context_trim(tpt_context* ctx) {
+  if (!ctx) return set_error(nullptr, TPT_ERR_INVALID_ARG, "NULL context");
+  if (tpt_status st = set_device(ctx)) return st;
+  void* block;
+  {
+    std::lock_guard<std::mutex> g(ctx->block_mu);
+    block = ctx->block;
+    ctx->block = nullptr;
+    ctx->block_bytes = 0;
+  }
+  if (block) cudaFree(block);
+  if (ctx->d_stage) cudaFree(ctx->d_stage);
+  ctx->d_stage = nullptr;
+  ctx->d_stage_bytes = 0;
+  if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
+  ctx->h_stage = nullptr;
+  ctx->h_stage_bytes = 0;
+  return TPT_OK;
+}
+
 // ---- host QBVH builder -----------------------------------------------------
 tpt_status tpt_qbvh_build(const float* bounds, uint64_t n, int threads, tpt_qbvh** out) {
   if (!out || (!bounds && n)) return set_error(nullptr, TPT_ERR_INVALID_ARG, "NULL argument");

@@ -281,6 +281,7 @@ EXPORTED_SYMBOLS = [
     "tpt_context_create",
     "tpt_context_destroy",
     "tpt_context_check",
+    "tpt_context_trim",
     "tpt_last_error",
     "tpt_version",
     "tpt_qbvh_build",
@@ -333,6 +334,7 @@ def _declare(L):
         "tpt_context_create": (i32, [i32, C.POINTER(vp)]),
         "tpt_context_destroy": (i32, [vp]),
         "tpt_context_check": (i32, [vp, vp]),
+        "tpt_context_trim": (i32, [vp]),
         "tpt_last_error": (cp, [vp]),
         "tpt_version": (cp, []),
         "tpt_qbvh_build": (i32, [vp, u64, i32, C.POINTER(vp)]),
@@ -419,6 +421,10 @@ class Context:
         """`tpt_context_check`: waits for `stream` and raises TptError when a
         device-side check of work queued by `*_device` calls fired."""
         _check(lib().tpt_context_check(self.h, _stream(stream)), self)
+
+    def trim(self):
+        """`tpt_context_trim`: gives back the memory kept for the next host-buffer call."""
+        _check(lib().tpt_context_trim(self.h), self)
 
     @property
     def wavefront_capacity(self) -> int:
