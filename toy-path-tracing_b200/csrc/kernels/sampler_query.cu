@@ -31,17 +31,17 @@ __global__ void sampler_values_kernel(uint32_t log2_spp, uint32_t n_digits, uint
   float v[16];
   ps.sample_2d(kDimCamera, v[0], v[1]);
   const uint32_t d = q.w;
+  // draws that a vertex makes together, as the render kernels make them
   v[2] = ps.sample_1d(vertex_dim(d, kOffCategory));
-  v[3] = ps.sample_1d(vertex_dim(d, kOffTree));
+  ps.sample_2d_1d(vertex_dim(d, kOffSurface), vertex_dim(d, kOffTree), v[5], v[6], v[3]);
   v[4] = ps.sample_1d(vertex_dim(d, kOffLightAux));
-  ps.sample_2d(vertex_dim(d, kOffSurface), v[5], v[6]);
-  v[7] = ps.sample_1d(vertex_dim(d, kOffLobe));
+  ps.sample_2d_1d(vertex_dim(d, kOffDir), vertex_dim(d, kOffLobe), v[9], v[10], v[7]);
   v[8] = ps.sample_1d(vertex_dim(d, kOffLayer));
-  ps.sample_2d(vertex_dim(d, kOffDir), v[9], v[10]);
-  v[11] = ps.sample_1d(vertex_dim(d, kOffExtra0));
-  v[12] = ps.sample_1d(vertex_dim(d, kOffExtra1));
-  v[13] = ps.sample_1d(vertex_dim(d, kOffExtra2));
-  v[14] = ps.sample_1d(vertex_dim(d, kOffExtra3));
+  const float4 extra = ps.sample_1d4(vertex_dim(d, kOffExtra0));
+  v[11] = extra.x;
+  v[12] = extra.y;
+  v[13] = extra.z;
+  v[14] = extra.w;
   v[15] = ps.sample_1d(vertex_dim(d, kOffRr));
 #pragma unroll
   for (int k = 0; k < 16; ++k) out[16 * i + k] = v[k];
