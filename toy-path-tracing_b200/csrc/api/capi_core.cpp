@@ -87,7 +87,7 @@ tpt_status CallBlock::take(size_t n) {
 
 CallBlock::~CallBlock() {
   if (!p) return;
-  cudaStreamSynchronize(stream);
+  if (!idle) cudaStreamSynchronize(stream);
   if (bytes <= kKeptBytes) {
     std::lock_guard<std::mutex> g(ctx->block_mu);
     if (bytes > ctx->block_bytes) {

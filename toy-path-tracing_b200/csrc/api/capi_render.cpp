@@ -333,19 +333,17 @@ struct ImageMemory {
     own = true;
     return cuda_check(block.ctx, cudaMallocAsync((void**)&p, bytes, block.stream), "cudaMallocAsync(image)");
   }
-  void give_back() {  // before the call's last synchronisation, which unmaps memory of its own
+  // The end of the call, after an error too: copies into the caller's images may be
+  // queued.  Memory of its own is freed first, so that the wait unmaps it.
+  tpt_status finish(tpt_status st) {
     if (own && p) cudaFreeAsync(p, block.stream);
     p = nullptr;
+    if (!st) st = check_device_errors(block.ctx, block.stream);
+    if (st) cudaStreamSynchronize(block.stream);
+    block.idle = true;
+    return st;
   }
 };
-
-// The end of a host-image render, after an error too: copies into the caller's
-// images may be queued.
-tpt_status finish_images(tpt_context* ctx, tpt_status st) {
-  if (!st) return check_device_errors(ctx, ctx->stream);
-  cudaStreamSynchronize(ctx->stream);
-  return st;
-}
 }  // namespace tpt
 
 extern "C" {
@@ -482,9 +480,7 @@ tpt_status tpt_render(tpt_context* ctx, const tpt_render_job* jobs, int n_jobs, 
       st = cuda_check(ctx, cudaMemcpyAsync(out_rgb[j], d[j], (size_t)jobs[j].width * jobs[j].height * 12,
                                            cudaMemcpyDeviceToHost, ctx->stream),
                       "D2H image");
-    mem.give_back();
-    st = finish_images(ctx, st);
-    return st;
+    return mem.finish(st);
   }
   for (int j = 0; j < n_jobs; ++j) {
     if (!out_rgb[j]) return set_error(ctx, TPT_ERR_INVALID_ARG, "NULL output image");
@@ -498,9 +494,7 @@ tpt_status tpt_render(tpt_context* ctx, const tpt_render_job* jobs, int n_jobs, 
     if (!st)
       st = cuda_check(ctx, cudaMemcpyAsync(out_rgb[j], mem.p, img_bytes, cudaMemcpyDeviceToHost, ctx->stream),
                       "D2H image");
-    mem.give_back();
-    st = finish_images(ctx, st);
-    if (st) return st;
+    if ((st = mem.finish(st))) return st;
   }
   return TPT_OK;
 }

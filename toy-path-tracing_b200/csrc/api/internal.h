@@ -140,13 +140,14 @@ void note_device_call(tpt_context* ctx, const char* name);
 // for the next call: mapping and unmapping memory costs a small call more than
 // its work.  A block belongs to one call at a time, so calls of several threads
 // do not share it (the larger of two given back is kept), and the destructor
-// waits for `stream` before giving it back, on error exits too.
+// waits for `stream` before giving it back (unless the call has), on error exits too.
 struct CallBlock {
   static constexpr size_t kKeptBytes = 128u << 20;  // a 4K image and more
   tpt_context* ctx;
   cudaStream_t stream;
   char* p = nullptr;
   size_t bytes = 0;
+  bool idle = false;  // `stream` has been waited for after the call's last work
   CallBlock(tpt_context* c, cudaStream_t s) : ctx(c), stream(s) {}
   CallBlock(const CallBlock&) = delete;
   ~CallBlock();
