@@ -117,8 +117,8 @@ tpt_status tpt_scene_set_openpbr(tpt_context* ctx, tpt_scene* scene, uint32_t co
     if (st) return st;
   }
   // one copy per run of consecutive table entries (in the list's order, so that
-  // a material listed twice keeps its last entry): each copy costs the host some
-  // 5 us
+  // a material listed twice keeps its last entry): a record's copy costs the host
+  // 1.7 us, 64 of them in one 3 to 16
   DevOpenPbr* table = const_cast<DevOpenPbr*>(scene->render.openpbr);
   for (uint32_t k = 0; k < count;) {
     const uint32_t t = scene->opbr_of_material[material_ids[k]];

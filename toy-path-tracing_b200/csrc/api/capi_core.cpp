@@ -158,8 +158,8 @@ struct HostCopies {
 };
 
 // Rows of `width` bytes between pitched buffers: one copy instead of one per row
-// (each costs the host some 3 us, a quarter of a small query's time), as far as the
-// driver's pitch limit of 2^31 - 1 bytes goes.
+// (16 KB rows from page-locked memory, one after another on a stream: 4.0 us each, six
+// of them in one copy 6.5 us), as far as the driver's pitch limit of 2^31 - 1 bytes goes.
 void copy_planes(void* dst, size_t dst_pitch, const void* src, size_t src_pitch, size_t width, size_t rows,
                  cudaMemcpyKind kind, cudaStream_t s) {
   if (std::max(dst_pitch, src_pitch) <= 0x7fffffffu) {

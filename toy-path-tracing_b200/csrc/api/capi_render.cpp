@@ -300,8 +300,9 @@ tpt_status render_bdpt_wavefront(tpt_context* ctx, const tpt_render_job* job, co
   return TPT_OK;
 }
 
-// Pixels per chunk: the per-sample buffer stays below 1 GiB and a chunk has at
-// most `capacity` paths (the wavefront arena's slot count; 0 = the default).
+// Pixels per chunk: at most `capacity` paths (the wavefront arena's slot count; 0 =
+// the default), and 1 GiB of samples where a buffer holds them (BDPT, the one-kernel
+// execution and the adjoint; no capacity reaches that limit today).
 uint32_t chunk_pixels(const RenderLaunch& L, uint32_t capacity) {
   if (capacity == 0) capacity = kDefaultWavefrontSlots;
   const uint64_t per_pixel = 12ull * L.spp;

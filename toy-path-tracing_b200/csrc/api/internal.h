@@ -232,7 +232,7 @@ cudaError_t launch_wf_generate(const DevGeometry& geo, const DevRenderData& rd, 
                                const WfBuffers& B, uint64_t first_path, uint32_t n_paths, cudaStream_t s,
                                const float* primal = nullptr);
 // shade reads the chunk's first path from the queue counters (written by generate)
-// `block`: threads per block of the (forward) shade stage, 128 or 256 (tpt_autotune picks it)
+// `block`: tpt_context_set_shade_block's setting, 128 or 256 (tpt_autotune picks it)
 cudaError_t launch_wf_shade(const DevGeometry& geo, const DevRenderData& rd, const RenderLaunch& P,
                             const WfBuffers& B, int cur, cudaStream_t s, const DevAdjoint* A = nullptr,
                             int block = 256);

@@ -25,8 +25,10 @@ namespace tpt {
 
 constexpr int kBlock = 128;
 constexpr int kShStack = 12;
-// Blocks per SM: 7 leave 72 registers, which the kernel fits without spilling
-// (8 blocks spill some 100 bytes a thread).
+// Blocks per SM: 7 leave 72 registers, into which queries without barycentrics fit;
+// renders (barycentrics) spill 8 bytes a thread, batches 38-66 stored and 100-116
+// loaded, counting and alpha-tested variants up to 106 and 140.  With 8 blocks the
+// plain query spills some 100.
 constexpr int kMinBlocks = 7;
 // Finished lanes that end the node phase early for a refill, and the lanes still
 // at interior nodes below which those waiting at a leaf go first: without the
