@@ -159,15 +159,21 @@ struct HostCopies {
 
 // Rows of `width` bytes between pitched buffers: one copy instead of one per row
 // (16 KB rows from page-locked memory, one after another on a stream: 4.0 us each, six
-// of them in one copy 6.5 us), as far as the driver's pitch limit of 2^31 - 1 bytes goes.
-void copy_planes(void* dst, size_t dst_pitch, const void* src, size_t src_pitch, size_t width, size_t rows,
-                 cudaMemcpyKind kind, cudaStream_t s) {
+// of them in one copy 6.5 us).  A copy of rows refuses what copies of one row take:
+// host memory that was page-locked in several pieces, or in part (a page-locked tensor
+// of an allocator that registers in pieces), and pitches above 2^31 - 1 bytes.
+cudaError_t copy_planes(void* dst, size_t dst_pitch, const void* src, size_t src_pitch, size_t width, size_t rows,
+                        cudaMemcpyKind kind, cudaStream_t s) {
+  cudaError_t e = cudaErrorInvalidValue;
   if (std::max(dst_pitch, src_pitch) <= 0x7fffffffu) {
-    cudaMemcpy2DAsync(dst, dst_pitch, src, src_pitch, width, rows, kind, s);
-    return;
+    e = cudaMemcpy2DAsync(dst, dst_pitch, src, src_pitch, width, rows, kind, s);
+    if (e == cudaErrorInvalidValue) cudaGetLastError();  // refused: nothing is queued
   }
-  for (size_t r = 0; r < rows; ++r)
-    cudaMemcpyAsync((char*)dst + r * dst_pitch, (const char*)src + r * src_pitch, width, kind, s);
+  if (e != cudaErrorInvalidValue) return e;
+  e = cudaSuccess;
+  for (size_t r = 0; e == cudaSuccess && r < rows; ++r)
+    e = cudaMemcpyAsync((char*)dst + r * dst_pitch, (const char*)src + r * src_pitch, width, kind, s);
+  return e;
 }
 
 tpt_status ensure_host_staging(tpt_context* ctx, size_t bytes) {
@@ -837,13 +843,15 @@ tpt_status tpt_traverse(tpt_context* ctx, const tpt_scene* scene, const float* r
   // Rays [b, b + m) of every plane, and of one output's planes
   const size_t pitch = n * 4;
   auto copy_in_planes = [&](uint64_t b, uint64_t m, const float* src, size_t src_pitch, cudaStream_t s) {
-    copy_planes(d_rays + b, pitch, src, src_pitch, m * 4, in_planes, cudaMemcpyHostToDevice, s);
+    return copy_planes(d_rays + b, pitch, src, src_pitch, m * 4, in_planes, cudaMemcpyHostToDevice, s);
   };
   auto copy_out_planes = [&](uint64_t b, uint64_t m, cudaStream_t s) {
+    cudaError_t e = cudaSuccess;
     for (const Out& o : outs)
-      if (o.host)
-        copy_planes((char*)o.host + b * 4, pitch, (const char*)o.dev + b * 4, pitch, m * 4, o.planes,
-                    cudaMemcpyDeviceToHost, s);
+      if (o.host && e == cudaSuccess)
+        e = copy_planes((char*)o.host + b * 4, pitch, (const char*)o.dev + b * 4, pitch, m * 4, o.planes,
+                        cudaMemcpyDeviceToHost, s);
+    return e;
   };
   if (in_pinned && out_pinned) {
     // Pinned buffers: copies in on one stream, kernels alternating on two
@@ -858,17 +866,18 @@ tpt_status tpt_traverse(tpt_context* ctx, const tpt_scene* scene, const float* r
     uint64_t b = 0;
     for (size_t c = 0; c < sizes.size(); ++c) {
       const uint64_t m = sizes[c];
-      copy_in_planes(b, m, rays + b, pitch, ctx->copy_in);
+      cudaError_t e = copy_in_planes(b, m, rays + b, pitch, ctx->copy_in);
+      if ((st = cuda_check(ctx, e, "copy of rays"))) return st;
       cudaEventRecord(ctx->ev_in[c], ctx->copy_in);
       cudaStream_t s = ctx->pipe[c & 1];
       cudaStreamWaitEvent(s, ctx->ev_in[c], 0);
-      cudaError_t e = launch_traverse_strided(scene->geo, d_rays + b, n, m, mode, d_prim + b, d_t + b,
-                                              d_inst ? d_inst + b : nullptr, d_bary ? d_bary + b : nullptr, n,
-                                              next_counter(ctx), ctx->d_err, ctx->num_sms, s, nullptr, nullptr);
+      e = launch_traverse_strided(scene->geo, d_rays + b, n, m, mode, d_prim + b, d_t + b,
+                                  d_inst ? d_inst + b : nullptr, d_bary ? d_bary + b : nullptr, n,
+                                  next_counter(ctx), ctx->d_err, ctx->num_sms, s, nullptr, nullptr);
       if ((st = cuda_check(ctx, e, "traverse kernel launch"))) return st;
       cudaEventRecord(ctx->ev_done[c], s);
       cudaStreamWaitEvent(ctx->copy_out, ctx->ev_done[c], 0);
-      copy_out_planes(b, m, ctx->copy_out);
+      if ((st = cuda_check(ctx, copy_out_planes(b, m, ctx->copy_out), "copy of results"))) return st;
       b += m;
     }
     cudaEventRecord(ctx->ev_slot[0], ctx->copy_out);
@@ -899,8 +908,9 @@ tpt_status tpt_traverse(tpt_context* ctx, const tpt_scene* scene, const float* r
     cudaStream_t s = ctx->pipe[c & 1];
     const uint64_t b = c * chunk, m = std::min<uint64_t>(chunk, n - b);
     float* hslot = slot_of(c);
+    cudaError_t e;
     if (in_pinned) {
-      copy_in_planes(b, m, rays + b, pitch, s);
+      e = copy_in_planes(b, m, rays + b, pitch, s);
     } else {
       // the slot's last chunk but one has been drained (or, with pinned results,
       // its event tells when its rays have been read)
@@ -908,17 +918,19 @@ tpt_status tpt_traverse(tpt_context* ctx, const tpt_scene* scene, const float* r
       HostCopies copies;
       for (int p = 0; p < in_planes; ++p) copies.add(hslot + p * m, rays + p * n + b, m * 4);
       copies.run();
-      copy_in_planes(b, m, hslot, m * 4, s);
+      e = copy_in_planes(b, m, hslot, m * 4, s);
     }
+    if ((st = cuda_check(ctx, e, "copy of rays"))) return st;
     // the kernel reads plane p of the chunk at d_rays + p*n + b: pass a view with stride n
-    cudaError_t e = launch_traverse_strided(scene->geo, d_rays + b, n, m, mode, d_prim + b, d_t + b,
-                                            d_inst ? d_inst + b : nullptr, d_bary ? d_bary + b : nullptr, n,
-                                            next_counter(ctx), ctx->d_err, ctx->num_sms, s, nullptr, nullptr);
+    e = launch_traverse_strided(scene->geo, d_rays + b, n, m, mode, d_prim + b, d_t + b,
+                                d_inst ? d_inst + b : nullptr, d_bary ? d_bary + b : nullptr, n, next_counter(ctx),
+                                ctx->d_err, ctx->num_sms, s, nullptr, nullptr);
     if ((st = cuda_check(ctx, e, "traverse kernel launch"))) return st;
     if (out_pinned)
-      copy_out_planes(b, m, s);
+      e = copy_out_planes(b, m, s);
     else  // the outputs' planes follow one another on the device
-      copy_planes(hslot + 7 * m, m * 4, d_prim + b, pitch, m * 4, n_out, cudaMemcpyDeviceToHost, s);
+      e = copy_planes(hslot + 7 * m, m * 4, d_prim + b, pitch, m * 4, n_out, cudaMemcpyDeviceToHost, s);
+    if ((st = cuda_check(ctx, e, "copy of results"))) return st;
     cudaEventRecord(ctx->ev_slot[c & 1], s);
     if (!out_pinned && c >= 1) drain(c - 1);
   }
