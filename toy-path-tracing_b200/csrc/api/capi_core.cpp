@@ -724,6 +724,8 @@ tpt_status tpt_scene_upload(tpt_context* ctx, const tpt_scene_desc* desc, tpt_sc
   s->geo.tlas_node_base = tlas_base;
   s->geo.tlas_root_word = tlas_root;
   s->geo.num_instances = desc->num_instances;
+  s->geo.num_nodes = (uint32_t)nodes.size();
+  s->geo.num_tris = (uint32_t)n_tris;
   st = upload_render_data(s, desc);
   // the copies are from pageable memory: the last bytes of each may reach the device
   // after it has returned, and the scene may be used on any stream from here on

@@ -63,6 +63,7 @@ struct DevGeometry {
   uint32_t tlas_node_base;
   uint32_t tlas_root_word;
   uint32_t num_instances;
+  uint32_t num_nodes, num_tris;  // of all levels and meshes: the bounds of traversal's reads
   uint32_t pad;
   // per instance: the opacity its material's alpha test compares an AuxRng
   // draw with (1: no alpha test); NULL when no instance has one

@@ -28,6 +28,13 @@
 // Hence 32-byte loads: four per node instead of seven, two per triangle instead
 // of three.  For the issue slots: packed two-lane subtracts and multiplies,
 // three-input min/max, and a branch-free ranking of the children.
+//
+// Every index that goes to memory is clamped to the scene's arrays (nodes,
+// triangles, instances).  The upload has checked the trees and a stack entry is
+// written before it is read, so no clamp changes an index; they make a read outside
+// the scene impossible whatever a ray or a word of the stack holds.  As minimum
+// instructions they cost nothing (2^24 incoherent rays 5.87 -> 5.85 ms, Cornell box
+// 1.88 -> 1.89, 2.1M-triangle scene 3.52 -> 3.53); as tests with an error flag 1-2 %.
 #pragma once
 #include "dev_types.cuh"
 
@@ -399,7 +406,7 @@ __device__ __forceinline__ void trav_init(const DevGeometry& G, TravState& s, fl
 template <bool STATS, class Stack>
 __device__ __forceinline__ void node_step(const DevGeometry& G, TravState& s, Stack& st, TraceCounters& cnt,
                                           uint32_t* err) {
-  const DevNode* n = G.nodes + s.node_base + s.next;
+  const DevNode* n = G.nodes + min(s.node_base + s.next, G.num_nodes - 1u);
   if (STATS) cnt.nodes++;
   float tmin[4];
   uint32_t ch[4];
@@ -451,9 +458,10 @@ __device__ __forceinline__ void leaf_step(const DevGeometry& G, TravState& s, St
   const uint32_t count = (w >> 24) & 0x7Fu, off = w & 0xFFFFFFu;
   if (s.in_blas) {
     // BLAS leaf: triangles in leaf order, t_max shrinking on each hit
-    if (!s.r.tris_ready) ray_setup_tris(s.r);
     uint32_t g = s.tri_base + off;
-    for (const uint32_t end = g + count; g != end; ++g) {
+    const uint32_t end = min(g + count, G.num_tris);
+    if (!s.r.tris_ready) ray_setup_tris(s.r);
+    for (; g < end; ++g) {
       const DevTri tri = load_tri(G.tris, g);
       if (STATS) cnt.tris++;
       float t, b0, b1, b2;
@@ -473,7 +481,7 @@ __device__ __forceinline__ void leaf_step(const DevGeometry& G, TravState& s, St
     }
     trav_pop(G, s, st);
   } else if (count == 0) {
-    enter_instance<ALPHA>(G, s, off);
+    enter_instance<ALPHA>(G, s, min(off, G.num_instances - 1u));
   } else {
     // TLAS leaf: its instances in order; the first is entered now
     if (s.sp + (int)count > kStackDepth) {
@@ -482,8 +490,8 @@ __device__ __forceinline__ void leaf_step(const DevGeometry& G, TravState& s, St
       s.next = kNone;
       return;
     }
-    for (int j = (int)count - 1; j >= 1; --j) st.set(s.sp++, kLeafBit | __ldg(G.tlas_prims + off + j));
-    enter_instance<ALPHA>(G, s, __ldg(G.tlas_prims + off));
+    for (int j = (int)count - 1; j >= 1; --j) st.set(s.sp++, kLeafBit | __ldg(G.tlas_prims + min(off + j, G.num_instances - 1u)));
+    enter_instance<ALPHA>(G, s, __ldg(G.tlas_prims + min(off, G.num_instances - 1u)));
   }
 }
 
