@@ -26,8 +26,8 @@ namespace tpt {
 constexpr int kBlock = 128;
 constexpr int kShStack = 12;
 // Blocks per SM: 7 leave 72 registers, into which queries without barycentrics fit;
-// renders (barycentrics) spill 8 bytes a thread, batches 38-66 stored and 100-116
-// loaded, counting and alpha-tested variants up to 106 and 140.  With 8 blocks the
+// renders (barycentrics) spill 8 bytes a thread, batches 78-110 stored and 120-136
+// loaded, counting and alpha-tested variants up to 146 and 160.  With 8 blocks the
 // plain query spills some 100.
 constexpr int kMinBlocks = 7;
 // Finished lanes that end the node phase early for a refill, and the lanes still
